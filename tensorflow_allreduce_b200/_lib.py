@@ -104,7 +104,8 @@ def _declare(lib):
         "bc_gru_supported": (i, [i, i, i, i, i]),
         "bc_gru_set_profile": (i, [vp]),
         "bc_gru_workspace_bytes": (ll, [i, i, i, i]),
-        "bc_gru_forward": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
+        "bc_gru_scratch_bytes": (ll, [i, i, i, i]),
+        "bc_gru_forward": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
         "bc_gru_backward": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
         "bc_bn_clip_forward": (i, [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, f, f, vp]),
         "bc_bn_clip_backward": (i, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, vp]),

@@ -148,18 +148,20 @@ int bc_emu_allgatherv(void* g, const void* const* ins, const unsigned long long*
 int bc_emu_barrier_probe(void* g, int absent, double timeout_s, void* stream);
 int bc_max_emulated_blocks(int device, int nranks);
 
-/* Persistent bidirectional GRU layer (tcgen05 / TMA kernels, csrc/cuda/gru_persistent.h). These
- * need no initialised group. All tensors fp32 on the current device; `workspace` =
- * bc_gru_workspace_bytes() bytes of scratch, `sync` = 256 zeroed uint32, `status` = 1 uint32 that
- * receives a non-zero code if a bounded wait ran out. `stream` is a cudaStream_t. */
+/* Persistent bidirectional GRU layer (tcgen05 kernels, csrc/cuda/gru_persistent.h). These need no
+ * initialised group. All tensors fp32 on the current device; the second pointer of a pair (direction 1) is
+ * unused when ndir == 1; `scratch` = bc_gru_scratch_bytes() bytes, zeroed when allocated and used by one call
+ * at a time; `status` = 1 uint32 that receives a non-zero code if a bounded wait ran out. `stream` is a
+ * cudaStream_t. bc_gru_workspace_bytes: the partial sums that one time step exchanges. */
 long long bc_gru_workspace_bytes(int T, int B, int H, int ndir);
+long long bc_gru_scratch_bytes(int T, int B, int H, int ndir);
 int bc_gru_supported(int device, int T, int B, int H, int ndir);
 /* Tuning aid: device buffer of 8 x T uint64 that block (0,0) of later launches fills with time stamps; NULL = off. */
 int bc_gru_set_profile(void* stamps);
-int bc_gru_forward(int T, int B, int H, int ndir, const float* w_hh, const float* b_hh, const float* gx, float* y, float* rsv,
-                   float* workspace, unsigned* sync, unsigned* status, double timeout_s, void* stream);
-int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh_t, const float* y, const float* rsv, const float* dy,
-                    float* dgx, float* dgh, float* workspace, unsigned* sync, unsigned* status, double timeout_s, void* stream);
+int bc_gru_forward(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* b_hh0, const float* b_hh1,
+                   const float* gx, float* y, float* rsv, void* scratch, unsigned* status, double timeout_s, void* stream);
+int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* y, const float* rsv,
+                    const float* dy, float* dg, float* db, void* scratch, unsigned* status, double timeout_s, void* stream);
 
 /* Training-mode batch normalisation of [N, C, HW] fp32 activations fused with the clipped ReLU behind it
  * (y = clamp(bn(x), 0, clip_hi)); csrc/cuda/bn_clip.h. `acc` = scratch of 2 * C doubles; running_* may be NULL.

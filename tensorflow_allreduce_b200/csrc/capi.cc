@@ -536,23 +536,31 @@ long long bc_gru_workspace_bytes(int T, int B, int H, int ndir) {
   return (long long)gpu::gru_persistent_workspace_bytes(d);
 }
 
-int bc_gru_forward(int T, int B, int H, int ndir, const float* w_hh, const float* b_hh, const float* gx, float* y, float* rsv,
-                   float* workspace, unsigned* sync, unsigned* status, double timeout_s, void* stream) {
+long long bc_gru_scratch_bytes(int T, int B, int H, int ndir) {
+  gpu::GruDims d{T, B, H, ndir};
+  return (long long)gpu::gru_persistent_scratch_bytes(d);
+}
+
+int bc_gru_forward(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* b_hh0, const float* b_hh1,
+                   const float* gx, float* y, float* rsv, void* scratch, unsigned* status, double timeout_s, void* stream) {
   API_BEGIN
   NvtxRange range("bcoll.gru_forward");
   gpu::GruDims d{T, B, H, ndir};
-  check_cuda(gpu::gru_persistent_forward(d, w_hh, b_hh, gx, y, rsv, workspace, sync, status, timeout_s, (cudaStream_t)stream),
+  const float* w[2] = {w_hh0, w_hh1};
+  const float* b[2] = {b_hh0, b_hh1};
+  check_cuda(gpu::gru_persistent_forward(d, w, b, gx, y, rsv, scratch, status, timeout_s, (cudaStream_t)stream),
              "persistent GRU forward launch");
   return 0;
   API_END(-1)
 }
 
-int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh_t, const float* y, const float* rsv, const float* dy,
-                    float* dgx, float* dgh, float* workspace, unsigned* sync, unsigned* status, double timeout_s, void* stream) {
+int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* y, const float* rsv,
+                    const float* dy, float* dg, float* db, void* scratch, unsigned* status, double timeout_s, void* stream) {
   API_BEGIN
   NvtxRange range("bcoll.gru_backward");
   gpu::GruDims d{T, B, H, ndir};
-  check_cuda(gpu::gru_persistent_backward(d, w_hh_t, y, rsv, dy, dgx, dgh, workspace, sync, status, timeout_s, (cudaStream_t)stream),
+  const float* w[2] = {w_hh0, w_hh1};
+  check_cuda(gpu::gru_persistent_backward(d, w, y, rsv, dy, dg, db, scratch, status, timeout_s, (cudaStream_t)stream),
              "persistent GRU backward launch");
   return 0;
   API_END(-1)

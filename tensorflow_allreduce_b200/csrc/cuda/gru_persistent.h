@@ -1,8 +1,8 @@
-// Persistent bidirectional GRU layer for sm_100a: the recurrent weights of a layer stay in shared
-// memory for all time steps, the per-step recurrent product runs on the 5th-generation tensor
-// cores (tcgen05.mma, TF32 operands, fp32 accumulator in tensor memory), operands arrive by TMA,
-// groups of blocks split the reduction length of the product among themselves, and the two
-// directions run side by side in one cooperative launch.
+// Persistent bidirectional GRU layer for sm_100a: the recurrent weights of a layer stay on chip (tensor
+// memory, and shared memory for what does not fit) for all time steps, the per-step recurrent product runs
+// on the 5th-generation tensor cores (tcgen05.mma, TF32 operands, fp32 accumulator), groups of blocks split
+// the reduction length of the product among themselves, and the two directions run side by side in one
+// cooperative launch.
 //
 // The reference's speech-model pieces are GRU cells that launch one GEMM plus elementwise
 // kernels per time step (tensorflow/contrib/rnn/kernels/gru_ops.h:69-119, gru_ops_gpu.cu.cc) or
@@ -31,42 +31,41 @@ struct GruDims {
 // Status bits written to status[0] by a block whose bounded wait ran out (the kernel then
 // returns early; outputs are incomplete).
 constexpr uint32_t kGruTimeoutGrid = 1u;      // waiting for the other blocks of its direction
-constexpr uint32_t kGruTimeoutCopy = 2u;      // waiting for a TMA copy
 constexpr uint32_t kGruTimeoutMma = 4u;       // waiting for the tensor core to finish
 
-// Forward. All tensors are fp32, contiguous, on the current device, 16-byte aligned.
-//   w_hh  [ndir, 3H, H]        recurrent weights
-//   b_hh  [ndir, 3H]
+// Forward. All tensors are fp32, contiguous, on the current device; w_hh, rsv and scratch 16-byte aligned.
+//   w_hh[dir] [3H, H]          recurrent weights of each direction
+//   b_hh[dir] [3H]
 //   gx    [T, B, ndir, 3H]     input projections including b_ih
-//   y     [T, B, ndir*H]       output (also read back as h_{t-1} by the next step)
-//   rsv   [ndir, T, B, 4, H]   r, z, n and (W_hn h + b_hn) of every step, for the backward pass
-//   workspace                  gru_persistent_workspace_bytes(d) bytes of scratch, zeroed once when it is
-//                              allocated and then reused as it is by every later call on the stream
-//   sync  [256] uint32         zero on entry; counters of the step and group barriers
+//   y     [T, B, ndir*H]       output
+//   rsv   [ndir, T, B, H, 4]   r, z, n and (W_hn h + b_hn) of every step, for the backward pass; may be null
+//   scratch                    gru_persistent_scratch_bytes(d) bytes, zeroed once when they are allocated and then reused
+//                              as they are by later calls, one after the other (concurrent calls need one each)
 //   status[1] uint32           ORed with kGruTimeout* on failure
 // `timeout_s` bounds every wait inside the kernel. Returns cudaErrorInvalidValue for unsupported
 // dimensions and cudaErrorCooperativeLaunchTooLarge if the grid cannot be co-resident.
-cudaError_t gru_persistent_forward(const GruDims& d, const float* w_hh, const float* b_hh, const float* gx, float* y, float* rsv,
-                                   float* workspace, uint32_t* sync, uint32_t* status, double timeout_s, cudaStream_t stream);
+cudaError_t gru_persistent_forward(const GruDims& d, const float* const* w_hh, const float* const* b_hh, const float* gx, float* y,
+                                   float* rsv, void* scratch, uint32_t* status, double timeout_s, cudaStream_t stream);
 
 // Backward through time.
-//   w_hh_t [ndir, H, 3H]       transposed recurrent weights
 //   y, rsv                     from the forward pass
 //   dy     [T, B, ndir*H]      gradient of the output
-//   dgx    [T, B, ndir, 3H]    out: gradient of gx                = (dr, dz, dn)
-//   dgh    [T, B, ndir, 3H]    out: gradient of (W_h h + b_h)     = (dr, dz, dn * r)
-// The caller forms dW_ih, dx, dW_hh and the bias gradients from dgx / dgh with library GEMMs.
-cudaError_t gru_persistent_backward(const GruDims& d, const float* w_hh_t, const float* y, const float* rsv, const float* dy,
-                                    float* dgx, float* dgh, float* workspace, uint32_t* sync, uint32_t* status, double timeout_s,
-                                    cudaStream_t stream);
+//   dg     [T, B, ndir*4H]     out: gradients of the pre-activations. Columns [0, ndir*3H): those of gx, (dr, dz, dn) of
+//                              direction 0, then of direction 1; columns ndir*3H + dir*H: dn * r. The gradient of
+//                              (W_h h + b_h) is (dr, dz, dn * r), so the two share their first two parts.
+//   db     [ndir, 2, 3H]       out: sums over time and batch of (dr, dz, dn) and of (dr, dz, dn * r): gradients of b_ih and b_hh
+// The caller forms dW_ih, dx and dW_hh from dg with library GEMMs.
+cudaError_t gru_persistent_backward(const GruDims& d, const float* const* w_hh, const float* y, const float* rsv, const float* dy,
+                                    float* dg, float* db, void* scratch, uint32_t* status, double timeout_s, cudaStream_t stream);
 
-// Bytes of scratch memory that a forward or backward call needs for these dimensions.
+// Bytes of partial sums that one step exchanges (plain fp32, the widest groups), and of scratch memory that
+// a forward or backward call needs for these dimensions.
 size_t gru_persistent_workspace_bytes(const GruDims& d);
+size_t gru_persistent_scratch_bytes(const GruDims& d);
 
-// Tuning aid: when `stamps` (device memory, 8 x T uint64) is non-null, block (0, 0) of every later
-// launch records %globaltimer at fixed points of each step: [0] step start, [1] peers' data
-// published, [2] first operand stage landed, [3] last MMA issued, [4] accumulator complete,
-// [5] gate math and stores done, [6] step published. Null switches it off.
+// Tuning aid: when `stamps` (device memory, 8 x T uint64) is non-null, thread 0 of block (0, 0) of every later
+// launch records %globaltimer at fixed points of each step: [0] step start, [1] operand in shared memory, [2] accumulator
+// complete, [3] partial sums sent, [4] partial sums received, [5] step published. Null switches it off.
 void gru_persistent_set_profile(unsigned long long* stamps);
 
 // True if this device and these dimensions can run the persistent kernels.
