@@ -30,18 +30,22 @@
 //     together depend on step s - 1 of EVERY block, and a block produces step s - 1 only after it
 //     has consumed all of step s - 2. Stale words of an earlier launch are cleared before the blocks
 //     of a direction meet once at the start.
+//   * Lines that another SM has just written are slow to read: 128 blocks that read 32 KB each take 1130 cycles
+//     when nothing was written, 1406 (the last block 1863) when it was. That is why the volume per block matters,
+//     why a loader thread reads 32 bytes per request, and why nothing is polled before it can be there.
 //   * Operand A from tensor memory: one M = 128, N = 32, K = 8 instruction takes 20 cycles, from shared
-//     memory 45 (it reads 5 KiB at 128 B per cycle). Weights that do not fit in the 512 columns
-//     (forward groups of four at H = 1024) stay in shared memory.
+//     memory 45 (it reads 5 KiB at 128 B per cycle). Weights that do not fit in the 512 columns stay in
+//     shared memory (forward pairs at H = 1024: 32 of 512 columns).
 //   * The MMAs are issued by an elected lane of a warp of its own; issued from under a
-//     `threadIdx.x == n` branch the same M = 64, N = 32 instruction took 55 cycles instead of 26.
-// One layer (T = 350, B = 32, H = 1024, both directions): see the figures at choose_split().
+//     `threadIdx.x == n` branch the same M = 64, N = 32 instruction took 55 cycles instead of 26. With two warps per
+//     scheduler every instruction of a serial chain costs four to six cycles, so the loops are kept short.
+//   * Two chains of half the batch each, meant to hide one's waits behind the other's work, were slower (4.7 us per step
+//     forward): what bounds the exchange is the fresh lines, not the number of bytes in flight.
+// Microseconds per step: see choose_split().
 //
 // Every wait is bounded by %globaltimer. When a wait runs out the block records a status bit, waits
 // (bounded) for its own MMAs in flight, frees its tensor memory and returns.
 #include "gru_persistent.h"
-
-#include <stdlib.h>
 
 #include <algorithm>
 #include <atomic>
@@ -53,12 +57,14 @@ namespace {
 
 constexpr int kUnits = 16;            // hidden units per block
 constexpr int kKTile = 32;            // fp32 elements in one 128-byte swizzle row
-constexpr int kWorkers = 256;         // eight warps: operand loads, accumulator read-back, exchange, gate math
-constexpr int kThreads = kWorkers + 32;   // plus the warp that issues the MMAs
+constexpr int kGateThreads = 256;     // eight warps: accumulator read-back, exchange, gate math
+constexpr int kLoadThreads = 256;     // eight warps: poll the operand words and put them into shared memory
+constexpr int kThreads = kGateThreads + kLoadThreads + 32;   // and the warp that issues the MMAs
 constexpr int kMaxBlocksPerDir = 64;  // H / 16 at H = 1024
 constexpr int kTmemCols = 512;
-constexpr int kLoadsPerGroup = 4;     // operand loads of a thread per pipeline group (one mbarrier each)
-constexpr int kMaxGroups = 7;         // of a step: 28 K tiles of 32 batch rows, H = 896 unsplit
+constexpr int kLoadBytes = kLoadThreads * 32;   // operand bytes that one load of every loader thread brings
+constexpr int kLoadsPerGroup = 2;     // loads of a thread per pipeline group (one mbarrier each)
+constexpr int kMaxGroups = 8;         // of a step: 32 K tiles of 32 batch rows, H = 1024 unsplit
 constexpr int kMinSmem = 120 * 1024;  // more than half of an SM's shared memory: one block per SM, since a block takes all of tensor memory
 
 struct Params {
@@ -71,7 +77,7 @@ struct Params {
   const float* dy;        // backward
   float* dg;              // backward: out
   float* db;              // backward: out
-  uint32_t* ring;         // operand words: [dir][slot 2][member C][K tile][batch B][32]
+  uint32_t* ring;         // operand words: [dir][slot 2][member C][K tile][batch NB][32]
   uint4* xchg;            // partial sums: [dir][owner block][source C][slot 2][pack][row] x 16 bytes
   uint32_t* sync;         // per direction: arrivals, generation
   uint32_t* status;
@@ -86,6 +92,11 @@ __device__ __forceinline__ unsigned long long gtimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
+}
+__device__ __forceinline__ uint32_t clock32() {
+  uint32_t c;
+  asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
+  return c;
 }
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
@@ -141,27 +152,23 @@ __device__ __forceinline__ void tc_mma_ss(uint32_t d, uint64_t adesc, uint64_t b
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// N consecutive columns of this thread's tensor-memory lane.
+// N consecutive columns of this thread's tensor-memory lane: the packs that one warp reads back (see `send` below).
 template <int N> __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t* r);
-template <> __device__ __forceinline__ void tc_ld<16>(uint32_t taddr, uint32_t* r) {
+template <> __device__ __forceinline__ void tc_ld<6>(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%6];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%4, %5}, [%7];\n\t"
       "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr) : "memory");
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5])
+      : "r"(taddr), "r"(taddr + 4) : "memory");
 }
-template <> __device__ __forceinline__ void tc_ld<32>(uint32_t taddr, uint32_t* r) {
+template <> __device__ __forceinline__ void tc_ld<9>(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%9];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x1.b32 {%8}, [%10];\n\t"
       "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr) : "memory");
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8])
+      : "r"(taddr), "r"(taddr + 8) : "memory");
 }
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const float* v) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
@@ -173,10 +180,17 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const float* v) {
 
 // Words that travel between blocks.
 __device__ __forceinline__ void st_word(uint32_t* p, uint32_t v) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
-__device__ __forceinline__ uint4 ld_words(const uint32_t* p) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
+// 32 bytes per request: a strong load costs L2 the same whatever its width (fresh lines, 32 KB per block and 128 blocks:
+// 1406 cycles this way, 1758 with 16-byte loads).
+struct Words { uint32_t w[8]; };
+// Two neighbouring chunks of a swizzled row: the second one's place differs in bit 4.
+__device__ __forceinline__ void st_shared2(uint32_t at, const Words& v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]), "r"(v.w[3]) : "memory");
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at ^ 16), "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]), "r"(v.w[7]) : "memory");
+}
+__device__ __forceinline__ void ld_words(const uint32_t* p, Words& v) {
+  asm volatile("ld.relaxed.gpu.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p) : "memory");
 }
 __device__ __forceinline__ void st_pack(uint4* p, uint4 v) {
   asm volatile(
@@ -196,8 +210,11 @@ __device__ __forceinline__ uint4 ld_pack(const uint4* p) {
 }
 constexpr uint32_t kTagMask = 0x1FFFu;
 __device__ __forceinline__ uint32_t tagged(float v, uint32_t tag) { return (__float_as_uint(v) & ~kTagMask) | tag; }
-__device__ __forceinline__ bool stale(const uint4& v, uint32_t tag) {
-  return (((v.x ^ tag) | (v.y ^ tag) | (v.z ^ tag) | (v.w ^ tag)) & kTagMask) != 0;
+__device__ __forceinline__ bool stale(const Words& v, uint32_t tag) {
+  uint32_t d = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) d |= v.w[i] ^ tag;
+  return (d & kTagMask) != 0;
 }
 
 // Shared-memory matrix descriptor of a K-major operand tile stored as rows of 128 bytes with the
@@ -212,30 +229,39 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
   return d;
 }
 
-__device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf(-x)); }
-
-// Barrier of the eight worker warps that also tells whether all of them are still fine.
-__device__ __forceinline__ bool workers_sync_and(bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %1, 0;\n\t"
-      "barrier.cta.red.and.pred q, 1, 256, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r) : "r"((uint32_t)ok) : "memory");
-  return r != 0;
+// The gate functions are on the critical path of every step and issue-bound (eight warps run 512 of each), so they are
+// made of the fewest instructions that keep fp32 accuracy: a reciprocal with one Newton step instead of a division.
+__device__ __forceinline__ float recip(float y) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return fmaf(r, fmaf(-y, r, 1.f), r);
 }
+__device__ __forceinline__ float sigmoidf_(float x) { return recip(1.f + __expf(fminf(-x, 80.f))); }
+// 1 - 2 / (1 + e^2x); near zero, where that cancels, the Taylor series up to x^9 (its error at 0.3 is 1e-8).
+__device__ __forceinline__ float tanhf_(float x) {
+  const float t = 1.f - 2.f * recip(1.f + __expf(fminf(2.f * x, 80.f)));
+  const float q = x * x;
+  float c = fmaf(q, 62.f / 2835.f, -17.f / 315.f);
+  c = fmaf(q, c, 2.f / 15.f);
+  c = fmaf(q, c, -1.f / 3.f);
+  return fabsf(x) < 0.3f ? fmaf(x * q, c, x) : t;
+}
+
+// Barrier 1: all gate and loader warps have read the accumulator and sent their part of it; the loaders only arrive.
+__device__ __forceinline__ void sent_sync() { asm volatile("barrier.cta.sync 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void sent_arrive() { asm volatile("barrier.cta.arrive 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void gates_sync() { asm volatile("barrier.cta.sync 2, 256;" ::: "memory"); }
 
 // Where everything of one block lives; a function of the pass, the split and the dimensions.
 struct Plan {
   int kq;            // K range of a member: columns of the recurrent weights it holds
   int ntile;         // K tiles of 32 (the last one may be half)
-  int m0, m1;        // M of the accumulator tiles (m1 = 0: one tile); rows beyond the group's are padding
-  int col0;          // first tensor-memory column of the weights; the accumulators lie below
-  int kt0, kt1;      // K columns of either tile that live in tensor memory; the others live in shared memory
+  int m;             // M of the MMAs: rows of the group, padded to 64 or 128
+  int k_tmem;        // K columns that live in tensor memory; the others live in shared memory
   int x_bytes, w_bytes, own_bytes;
   __host__ __device__ int smem() const { return 1024 + x_bytes + w_bytes + own_bytes + 256; }
 };
+__host__ __device__ constexpr int packs_of(int batch) { return (batch + 2) / 3; }   // three partial sums and the step number per 16 bytes
 template <bool BWD> struct RowsPerOwner { static constexpr int value = BWD ? kUnits : 3 * kUnits; };
 
 template <bool BWD>
@@ -244,19 +270,14 @@ __host__ __device__ inline Plan make_plan(int C, int nb, int H) {
   const int rows = RowsPerOwner<BWD>::value * C;
   p.kq = (BWD ? 3 * H : H) / C;
   p.ntile = (p.kq + kKTile - 1) / kKTile;
-  p.m0 = rows > 64 ? 128 : 64;
-  p.m1 = rows > 128 ? (rows > 192 ? 128 : 64) : 0;
-  p.col0 = p.m1 ? 2 * nb : nb;
-  int room = kTmemCols - p.col0;
-  p.kt0 = p.kq <= room ? p.kq : room / kKTile * kKTile;
-  room -= p.kt0;
-  p.kt1 = !p.m1 ? 0 : p.kq <= room ? p.kq : room / kKTile * kKTile;
+  p.m = rows > 64 ? 128 : 64;
+  const int room = kTmemCols - nb;                 // the accumulator takes the first nb columns
+  p.k_tmem = p.kq <= room ? p.kq : room / kKTile * kKTile;
   p.x_bytes = p.ntile * nb * 128;
-  p.w_bytes = ((p.kq - p.kt0 + kKTile - 1) / kKTile * p.m0 + (p.m1 ? (p.kq - p.kt1 + kKTile - 1) / kKTile * p.m1 : 0)) * 128;
-  p.own_bytes = RowsPerOwner<BWD>::value * (nb + 1) * 4;
+  p.w_bytes = (p.kq - p.k_tmem + kKTile - 1) / kKTile * p.m * 128;
+  p.own_bytes = RowsPerOwner<BWD>::value * packs_of(nb) * 16;
   return p;
 }
-__host__ __device__ inline int packs_of(int batch) { return (batch + 2) / 3; }   // three partial sums and the step number per 16 bytes
 
 // The 16 weights of row `r` of the group at columns k0 .. k0 + 15 of member q's K range (k0 a multiple of 16).
 //   forward : rows ordered owner, gate, unit; K = hidden units            W[g * H + unit][q * kq + k]
@@ -277,28 +298,12 @@ __device__ __forceinline__ void load_weights16(const float* w, int H, int C, int
   }
 }
 
-// Inputs of one backward step for the (unit, batch) pairs of a thread.
-struct BwdInputs {
-  float4 a[3];          // r, z, n, W_hn h + b_hn
-  float hp[3], dy[3];
-};
-
-__device__ __forceinline__ void load_bwd_inputs(const Params& p, BwdInputs& in, int t, int dir, int unit, int b0, int nb) {
-  const int T = p.d.T, B = p.d.B, H = p.d.H, ND = p.d.ndir;
-  const int tprev = dir ? t + 1 : t - 1;
-  const bool has_prev = tprev >= 0 && tprev < T;
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    if (j < nb) {
-      const int b = b0 + j;
-      in.a[j] = __ldg(p.rsv + ((size_t)(dir * T + t) * B + b) * H + unit);
-      in.hp[j] = has_prev ? __ldg(p.y + ((size_t)tprev * B + b) * (ND * H) + dir * H + unit) : 0.f;
-      in.dy[j] = __ldg(p.dy + ((size_t)t * B + b) * (ND * H) + dir * H + unit);
-    }
-  }
-}
-
 // BWD: pass; C: blocks per group; NB: N of the MMA (16 or 32, at least the batch).
+//
+// Three kinds of warps, so that no work off the chain of a step (output stores, prefetches) delays the next
+// product: gate warps, loader warps, and one warp that issues the MMAs. One barrier each says that
+// the operand is in shared memory (full[group]: loaders -> MMA), that the accumulator is complete (done:
+// MMA -> all), that it has been read (read: all -> MMA), and that this block has published (published: gates -> loaders).
 template <bool BWD, int C, int NB>
 __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -308,7 +313,6 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
   constexpr int kRows = RowsPerOwner<BWD>::value;
   constexpr int R = kRows * C;
   constexpr int kGates = BWD ? 1 : 3;      // accumulator rows per unit
-  constexpr int kOwnStride = NB + 1;
   constexpr int kGateWords = BWD ? 3 : 1;  // operand words that a (unit, batch) pair publishes per step
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dir = blockIdx.y, u0 = blockIdx.x * kUnits;
@@ -320,21 +324,23 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
 
   uint8_t* x_s = smem;
   uint8_t* w_s = smem + pl.x_bytes;
-  float* own_s = reinterpret_cast<float*>(w_s + pl.w_bytes);                       // this block's own rows of the accumulator
-  uint64_t* bar_s = reinterpret_cast<uint64_t*>(w_s + pl.w_bytes + pl.own_bytes);  // full[kMaxGroups], done, drain
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_s + kMaxGroups + 2);
+  uint4* own_s = reinterpret_cast<uint4*>(w_s + pl.w_bytes);                       // this block's own partial sums: [pack][row]
+  uint64_t* bar_s = reinterpret_cast<uint64_t*>(w_s + pl.w_bytes + pl.own_bytes);  // full[kMaxGroups], done, drain, read, published
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_s + kMaxGroups + 4);
   volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const uint32_t full_bar = smem_u32(bar_s), done_bar = full_bar + 8 * kMaxGroups, drain_bar = done_bar + 8;
+  const uint32_t full_bar = smem_u32(bar_s), done_bar = full_bar + 8 * kMaxGroups, drain_bar = done_bar + 8, read_bar = done_bar + 16, pub_bar = done_bar + 24;
   const uint32_t x_addr = smem_u32(x_s), w_addr = smem_u32(w_s);
 
   if (tid == 0) {
-    for (int i = 0; i < kMaxGroups; i++) mbar_init(full_bar + 8 * i, kWorkers / 32);
+    for (int i = 0; i < kMaxGroups; i++) mbar_init(full_bar + 8 * i, kLoadThreads / 32);
     mbar_init(done_bar, 1);
     mbar_init(drain_bar, 1);
+    mbar_init(read_bar, (kGateThreads + kLoadThreads) / 32);
+    mbar_init(pub_bar, kGateThreads / 32);
     *abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kWorkers / 32) {
+  if (warp == kThreads / 32 - 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -342,7 +348,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
   // The part of the ring that this block writes (both slots) and the partial sums that it will
   // receive: cleared, so that nothing of an earlier launch passes for a word of this one.
   const int range = H / C;                                       // units of one member's K range
-  const uint32_t ring_member = (uint32_t)pl.ntile * B * kKTile;  // words of one member's range and slot
+  const uint32_t ring_member = (uint32_t)pl.ntile * NB * kKTile;  // words of one member's range and slot
   const uint32_t ring_slot = ring_member * C;
   uint32_t* ring = p.ring + (size_t)dir * 2 * ring_slot;
   // word of (gate g, unit u0 + u, batch b): member u0 / range, column g * range + u0 % range + u
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
   const int my_col = u0 % range;
   auto ring_at = [&](int g, int u, int b) -> uint32_t {
     const int k = g * range + my_col + u;
-    return my_member + (uint32_t)((k >> 5) * B + b) * kKTile + (k & 31);
+    return my_member + (uint32_t)((k >> 5) * NB + b) * kKTile + (k & 31);
   };
   const int xslot = npacks * kRows;                              // 16-byte words of one tile and slot
   uint4* xin = p.xchg + ((size_t)dir * nblocks + blockIdx.x) * C * 2 * xslot;
@@ -381,41 +387,32 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     }
   }
 
-  // The group's weight rows for this block's K range, resident for the whole sequence. In a tile with
-  // M = 128 row r is lane r of tensor memory; with M = 64 it is lane (r / 16) * 32 + r % 16.
+  // The group's weight rows for this block's K range, resident for the whole sequence. With M = 128 row r is
+  // lane r of tensor memory; with M = 64 it is lane (r / 16) * 32 + r % 16, the other lanes are not used.
   const float* w = p.w_hh[dir];
-  if (warp < kWorkers / 32) {
-    const int quarter = warp & 3;
-    for (int tile = 0; tile < (pl.m1 ? 2 : 1); tile++) {
-      const int m = tile ? pl.m1 : pl.m0, kt = tile ? pl.kt1 : pl.kt0;
-      const int r = tile * 128 + (m == 128 ? quarter * 32 + lane : quarter * 16 + (lane & 15));
-      const bool valid = r < R && (m == 128 || lane < 16);
-      for (int k0 = 16 * (warp >> 2); k0 < kt; k0 += 32) {
-        float v[16];
+  const int quarter = warp & 3;
+  const int lane_row = pl.m == 128 ? quarter * 32 + lane : quarter * 16 + (lane & 15);
+  const bool row_ok = lane_row < R && (pl.m == 128 || lane < 16);
+  if (warp < 8) {
+    for (int k0 = 16 * (warp >> 2); k0 < pl.k_tmem; k0 += 32) {
+      float v[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) v[i] = 0.f;
-        if (valid) load_weights16<BWD>(w, H, C, grp, q, pl.kq, r, k0, v);
-        __syncwarp();
-        tc_st16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(pl.col0 + (tile ? pl.kt0 : 0) + k0), v);
-      }
+      for (int i = 0; i < 16; i++) v[i] = 0.f;
+      if (row_ok) load_weights16<BWD>(w, H, C, grp, q, pl.kq, lane_row, k0, v);
+      __syncwarp();
+      tc_st16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(NB + k0), v);
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-    uint8_t* dst = w_s;
-    for (int tile = 0; tile < (pl.m1 ? 2 : 1); tile++) {
-      const int m = tile ? pl.m1 : pl.m0, kt = tile ? pl.kt1 : pl.kt0;
-      const int runs = (pl.kq - kt) / 16;
-      for (int i = tid; i < m * runs; i += kWorkers) {
-        const int rt = i % m, r = tile * 128 + rt, k = (i / m) * 16;      // counted from kt
-        float v[16];
+    for (int i = tid; i < pl.m * ((pl.kq - pl.k_tmem) / 16); i += 256) {
+      const int r = i % pl.m, k = (i / pl.m) * 16;                     // counted from k_tmem
+      float v[16];
 #pragma unroll
-        for (int e = 0; e < 16; e++) v[e] = 0.f;
-        if (r < R) load_weights16<BWD>(w, H, C, grp, q, pl.kq, r, kt + k, v);
-        uint8_t* row = dst + ((k >> 5) * m + rt) * 128;
+      for (int e = 0; e < 16; e++) v[e] = 0.f;
+      if (r < R) load_weights16<BWD>(w, H, C, grp, q, pl.kq, r, pl.k_tmem + k, v);
+      uint8_t* row = w_s + ((k >> 5) * pl.m + r) * 128;
 #pragma unroll
-        for (int e = 0; e < 4; e++)
-          reinterpret_cast<float4*>(row)[(((k & 31) >> 2) + e) ^ (rt & 7)] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-      }
-      dst += (runs + 1) / 2 * m * 128;
+      for (int e = 0; e < 4; e++)
+        reinterpret_cast<float4*>(row)[(((k & 31) >> 2) + e) ^ (r & 7)] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
     }
     fence_proxy_async();
   }
@@ -436,117 +433,136 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
   ok = __syncthreads_and(ok) != 0;
   tc_fence_after();
 
-  const int nrows = pl.ntile * B;                                // operand rows (K tile, batch entry) of 128 bytes
-  const int ngroups = (nrows + 32 * kLoadsPerGroup - 1) / (32 * kLoadsPerGroup);
+  // A loader thread's load `it` is the 32-byte word lt + 256 it of the member's range, i.e. chunks 2 (lt % 4) and the next
+  // of batch row lt / 4 % NB in K tile it * (64 / NB) + lt / 4 / NB: 8 KiB further per load in the ring and in shared memory.
+  constexpr int kTilesPerLoad = 64 / NB;
+  const int nloads = (pl.ntile + kTilesPerLoad - 1) / kTilesPerLoad;
+  const int ngroups = (nloads + kLoadsPerGroup - 1) / kLoadsPerGroup;
+  auto give_up = [&](uint32_t why) {
+    atomicOr(p.status, why);
+    *abort_s = 1;
+    return false;
+  };
 
-  if (ok && warp == kWorkers / 32) {
+  // Read-back of the accumulator, by gate and loader warps together: a warp may read the quarter warp % 4 of the lanes, and
+  // the four warps of a quarter share the packs of its rows (three batch entries each).
+  constexpr int kPacks = packs_of(NB), kPart = (kPacks + 3) / 4;
+  const int owner = lane_row / kRows, rr = lane_row % kRows;
+  const int pk_lo = (warp >> 2) * kPart, pk_n = max(0, min(kPart, npacks - pk_lo));
+  uint4* xout = p.xchg + (((size_t)dir * nblocks + grp * C + owner) * C + q) * 2 * xslot + pk_lo * kRows + rr;
+  auto send = [&](uint32_t tag, uint32_t parity) {
+    uint32_t v[3 * kPart];
+    tc_fence_after();
+    // a few columns past the accumulator's are read as well (they are inside the allocation) and sent as padding
+    tc_ld<3 * kPart>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(3 * pk_lo), v);
+    tc_fence_before();
+    if (lane == 0) mbar_arrive(read_bar);
+    if (row_ok) {
+      if (owner == q) {
+#pragma unroll
+        for (int i = 0; i < kPart; i++)
+          if (i < pk_n) own_s[(pk_lo + i) * kRows + rr] = make_uint4(v[3 * i], v[3 * i + 1], v[3 * i + 2], 0);
+      } else {
+        uint4* o = xout + (parity ? xslot : 0);
+#pragma unroll
+        for (int i = 0; i < kPart; i++)
+          if (i < pk_n) st_pack(o + i * kRows, make_uint4(v[3 * i], v[3 * i + 1], v[3 * i + 2], tag));
+      }
+    }
+  };
+
+  if (ok && warp == kThreads / 32 - 1) {
     // ---------------- the warp that issues the MMAs ----------------
     const bool leader = elect_one();
     const uint32_t fmt = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NB >> 3) << 17);
-    const uint32_t idesc0 = fmt | ((uint32_t)(pl.m0 >> 4) << 24), idesc1 = fmt | ((uint32_t)(pl.m1 >> 4) << 24);
-    const uint64_t b_desc = operand_desc(x_addr);
-    const uint64_t a_desc0 = operand_desc(w_addr);
-    const uint64_t a_desc1 = operand_desc(w_addr + (pl.kq - pl.kt0 + kKTile - 1) / kKTile * pl.m0 * 128);
-    const uint32_t d0 = tmem, d1 = tmem + NB, a0 = tmem + pl.col0, a1 = a0 + pl.kt0;
+    const uint32_t idesc = fmt | ((uint32_t)(pl.m >> 4) << 24);
+    const uint64_t b_desc = operand_desc(x_addr), a_desc = operand_desc(w_addr);
+    const uint32_t a_tmem = tmem + NB;
+    const int full_tiles = pl.kq / kKTile;              // and perhaps half a tile behind them
+    const int ts = pl.k_tmem / kKTile;                  // full K tiles whose weights are in tensor memory
+    constexpr uint32_t kBStep = NB * 128 / 16;          // descriptor units from one K tile to the next
+    const uint32_t a_step = (uint32_t)pl.m * 128 / 16;
     for (int s = 1; ok && s < T; s++) {
-      int done_tiles = 0;
-      for (int g = 0; ok && g < ngroups; g++) {
-        ok = mbar_wait(full_bar + 8 * g, (uint32_t)(s - 1) & 1, 4 * p.timeout_ns, abort_s);
+      if (s > 1) ok = mbar_wait(read_bar, (uint32_t)s & 1, 4 * p.timeout_ns, abort_s);
+      for (int g = 0; g < ngroups; g++) {
+        ok = ok && mbar_wait(full_bar + 8 * g, (uint32_t)(s - 1) & 1, 4 * p.timeout_ns, abort_s);
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (!ok) break;
         tc_fence_after();
-        const int have = min(kLoadsPerGroup * 32 * (g + 1), nrows) / B;
         if (leader) {
-          for (int kt = done_tiles; kt < have; kt++) {
-            const int steps = min(4, (pl.kq - kt * kKTile) / 8);
-            const uint64_t b = b_desc + (uint64_t)(kt * NB * 128 >> 4);
-            const int k0 = kt * kKTile;
-            if (k0 < pl.kt0) {
+          const int lo = g * kLoadsPerGroup * kTilesPerLoad, hi = min(full_tiles, lo + kLoadsPerGroup * kTilesPerLoad);
+          uint64_t b = b_desc + (uint64_t)((uint32_t)lo * kBStep);
+          uint32_t acc = lo > 0, a = a_tmem + lo * kKTile;
+          int kt = lo;
+#pragma unroll 2
+          for (; kt < min(hi, ts); kt++) {
 #pragma unroll
-              for (int ks = 0; ks < 4; ks++)
-                if (ks < steps) tc_mma_ts(d0, a0 + k0 + 8 * ks, b + 2 * ks, idesc0, kt + ks > 0);
-            } else {
-              const uint64_t a = a_desc0 + (uint64_t)((k0 - pl.kt0) / kKTile * pl.m0 * 128 >> 4);
-#pragma unroll
-              for (int ks = 0; ks < 4; ks++)
-                if (ks < steps) tc_mma_ss(d0, a + 2 * ks, b + 2 * ks, idesc0, kt + ks > 0);
+            for (int ks = 0; ks < 4; ks++) {
+              tc_mma_ts(tmem, a + 8 * ks, b + 2 * ks, idesc, acc);
+              acc = 1;
             }
-            if (R > 128) {
-              if (k0 < pl.kt1) {
+            a += kKTile;
+            b += kBStep;
+          }
+          uint64_t as = a_desc + (uint64_t)((uint32_t)max(0, kt - ts) * a_step);
+          for (; kt < hi; kt++) {
 #pragma unroll
-                for (int ks = 0; ks < 4; ks++)
-                  if (ks < steps) tc_mma_ts(d1, a1 + k0 + 8 * ks, b + 2 * ks, idesc1, kt + ks > 0);
-              } else {
-                const uint64_t a = a_desc1 + (uint64_t)((k0 - pl.kt1) / kKTile * pl.m1 * 128 >> 4);
+            for (int ks = 0; ks < 4; ks++) {
+              tc_mma_ss(tmem, as + 2 * ks, b + 2 * ks, idesc, acc);
+              acc = 1;
+            }
+            as += a_step;
+            b += kBStep;
+          }
+          if (g == ngroups - 1) {
+            if (full_tiles < pl.ntile) {
 #pragma unroll
-                for (int ks = 0; ks < 4; ks++)
-                  if (ks < steps) tc_mma_ss(d1, a + 2 * ks, b + 2 * ks, idesc1, kt + ks > 0);
+              for (int ks = 0; ks < 2; ks++) {
+                if (full_tiles * kKTile < pl.k_tmem) tc_mma_ts(tmem, a_tmem + full_tiles * kKTile + 8 * ks, b + 2 * ks, idesc, full_tiles + ks > 0);
+                else tc_mma_ss(tmem, as + 2 * ks, b + 2 * ks, idesc, full_tiles + ks > 0);
               }
             }
+            tc_commit(done_bar);
           }
-          if (g == ngroups - 1) tc_commit(done_bar);
         }
-        done_tiles = have;
         __syncwarp();
       }
     }
     if (!ok && leader) {
-      // A wait ran out here or in a worker. Nothing may be in flight when tensor memory is freed.
+      // A wait ran out here or in another warp. Nothing may be in flight when tensor memory is freed.
       *abort_s = 1;
       tc_commit(drain_bar);
       mbar_wait(drain_bar, 0, p.timeout_ns, nullptr);
     }
     __syncwarp();
-  } else if (ok) {
-    // ---------------- the workers ----------------
-    // Worker (u, pk) handles unit u0 + u for the batch entries b0 .. b0 + mine - 1.
-    const int u = tid & 15, pk = tid >> 4, b0 = 3 * pk;
-    const int mine = pk < npacks ? min(3, B - b0) : 0;
-    float carry[3] = {0.f, 0.f, 0.f};   // forward: h_{t-1}; backward: recurrent part of dh_t
-    // Operand load `it` of this thread: 16-byte word tid + 256 it of the member's range, i.e. chunk tid % 8 of
-    // row tid / 8 + 32 it = (K tile, batch entry). Its place in shared memory, or -1 if there is none:
-    const int chunk = tid & 7, row0 = tid >> 3;
+  } else if (ok && warp >= kGateThreads / 32) {
+    // ---------------- loaders ----------------
+    const int lt = tid - kGateThreads, chunk = 2 * (lt & 3), row = lt >> 2, b = row & (NB - 1), kt0 = row / NB;
     const int last_chunks = (pl.kq - (pl.ntile - 1) * kKTile) / 4;      // valid chunks of the last K tile
-    const int inv_b = 65536 / B + 1;                                  // row / B for row < 2048
-    auto place = [&](int it) -> int {
-      const int row = row0 + 32 * it, kt = (row * inv_b) >> 16, b = row - kt * B;
-      return (row < nrows && (kt < pl.ntile - 1 || chunk < last_chunks)) ? (kt * NB + b) * 128 + ((chunk ^ (b & 7)) << 4) : -1;
-    };
-    const uint32_t* src0 = ring + (size_t)q * ring_member + (size_t)tid * 4;
-    constexpr bool two_tiles = R > 128;
-    const int quarter = warp & 3, tile = two_tiles ? warp >> 2 : 0, m = tile ? pl.m1 : pl.m0;
-    const int r = tile * 128 + (m == 128 ? quarter * 32 + lane : quarter * 16 + (lane & 15));   // row of the accumulator
-    const bool row_ok = r < R && (m == 128 || lane < 16);
-    const int owner = r / kRows, rr = r % kRows;
-    constexpr int kPacks = (NB + 2) / 3, kHalf = (kPacks + 1) / 2;
-    // one tile: the first four warps take the first half of the packs, the others the rest
-    const int pk_lo = two_tiles || warp < 4 ? 0 : kHalf, pk_hi = min(npacks, two_tiles || warp >= 4 ? kPacks : kHalf);
-    uint4* xout = p.xchg + (((size_t)dir * nblocks + grp * C + owner) * C + q) * 2 * xslot + rr;
-    const bool stamping = p.prof && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0;
-    auto stamp = [&](int s, int i) {
-      if (stamping) p.prof[(size_t)s * 8 + i] = gtimer();
-    };
-    auto give_up = [&](uint32_t why) {
-      atomicOr(p.status, why);
-      *abort_s = 1;
-      return false;
-    };
-
-    // One recurrent product: the operand words tagged `tag`, the MMAs, the exchange inside the group.
-    // acc[g][j] receives the sum of this thread's unit (forward: gate g) for batch entry b0 + j.
-    // `good` falls when one of this thread's waits has run out; every worker comes through workers_sync_and() all the
-    // same, where all of them learn of it (the result is false then).
-    auto product = [&](uint32_t tag, int s, float (*acc)[3], bool& good) -> bool {
-      const uint32_t parity = (tag - 1) & 1;
+    const uint32_t dst = x_addr + (uint32_t)(row * 128 + ((chunk ^ (b & 7)) << 4));
+    const uint32_t* src0 = ring + (size_t)q * ring_member + (size_t)lt * 8;
+    // loads of this thread: K tiles kt0, kt0 + kTilesPerLoad, ... below ntile, the last one only if it has these chunks
+    const int tiles_mine = chunk < last_chunks ? pl.ntile : pl.ntile - 1;
+    const int mine = b < B && kt0 < tiles_mine ? (tiles_mine - kt0 + kTilesPerLoad - 1) / kTilesPerLoad : 0;
+    const uint32_t pause = (uint32_t)(pl.ntile * B * 128) / 80;      // cycles
+    constexpr int kSpan = 3;           // groups whose loads are in flight together
+    bool good = true;
+    // Every step is gone through to the end even when a wait has run out (the waits then end at once): the gate warps count
+    // on the arrivals.
+    for (int s = 1; s < T; s++) {
+      const uint32_t tag = (uint32_t)s, parity = (uint32_t)(s - 1) & 1;
       const uint32_t* src = src0 + (size_t)parity * ring_slot;
-      constexpr int kSpan = 3;           // groups whose loads are in flight together
+      // Not before this block has published its own words of the step, and then only when the others' are about to
+      // arrive: polling takes L2 bandwidth from the blocks that still exchange partial sums. (Backward, H = 1024, B = 32:
+      // polling all the time 6.8 us per step, from the publication on 4.75 us, with the pause 4.4 us.)
+      good = good && mbar_wait(pub_bar, parity, 4 * p.timeout_ns, abort_s);
+      for (const uint32_t c0 = clock32(); clock32() - c0 < pause;) {
+      }
       for (int g0 = 0; g0 < ngroups; g0 += kSpan) {
-        uint4 v[kSpan * kLoadsPerGroup];
+        Words v[kSpan * kLoadsPerGroup];
 #pragma unroll
-        for (int i = 0; i < kSpan * kLoadsPerGroup; i++) {
-          const int it = g0 * kLoadsPerGroup + i;
-          if (place(it) >= 0) v[i] = ld_words(src + (size_t)it * (kWorkers * 4));
-        }
+        for (int i = 0; i < kSpan * kLoadsPerGroup; i++)
+          if (g0 * kLoadsPerGroup + i < mine) ld_words(src + (g0 * kLoadsPerGroup + i) * (kLoadBytes / 4), v[i]);
 #pragma unroll
         for (int gi = 0; gi < kSpan; gi++) {
           if (g0 + gi < ngroups) {
@@ -556,10 +572,9 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
               bool missing = false;
 #pragma unroll
               for (int i = gi * kLoadsPerGroup; i < (gi + 1) * kLoadsPerGroup; i++) {
-                const int it = g0 * kLoadsPerGroup + i;
-                if (place(it) >= 0 && stale(v[i], tag)) {
+                if (g0 * kLoadsPerGroup + i < mine && stale(v[i], tag)) {
                   missing = true;
-                  v[i] = ld_words(src + (size_t)it * (kWorkers * 4));
+                  ld_words(src + (g0 * kLoadsPerGroup + i) * (kLoadBytes / 4), v[i]);
                 }
               }
               if (!missing || !good) break;
@@ -571,57 +586,63 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
               }
             }
 #pragma unroll
-            for (int i = gi * kLoadsPerGroup; i < (gi + 1) * kLoadsPerGroup; i++) {
-              const int at = place(g0 * kLoadsPerGroup + i);
-              if (at >= 0) *reinterpret_cast<uint4*>(x_s + at) = v[i];
-            }
+            for (int i = gi * kLoadsPerGroup; i < (gi + 1) * kLoadsPerGroup; i++)
+              if (g0 * kLoadsPerGroup + i < mine)
+                st_shared2(dst + (g0 * kLoadsPerGroup + i) * kLoadBytes, v[i]);
             fence_proxy_async();
-            tc_fence_before();           // this thread's reads of the previous accumulator come before the MMAs
             __syncwarp();
             if (lane == 0) mbar_arrive(full_bar + 8 * (g0 + gi));
           }
         }
       }
+      // The MMAs have read the operand area and written the accumulator.
+      if (good && !mbar_wait(done_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutMma);
+      if (__all_sync(0xffffffffu, good)) send(tag, parity);
+      else good = false;
+      sent_arrive();
+    }
+  } else if (ok) {
+    // ---------------- gates ----------------
+    // Thread (u, pk) handles unit u0 + u for the batch entries b0 .. b0 + mine - 1.
+    const int u = tid & 15, pk = tid >> 4, b0 = 3 * pk;
+    const int mine = pk < npacks ? min(3, B - b0) : 0;
+    float carry[3] = {0.f, 0.f, 0.f};   // forward: h_{t-1}; backward: recurrent part of dh_t
+    const uint4* xmine = xin + pk * kRows + u;
+    const uint4* own_mine = own_s + pk * kRows + u;
+    const bool stamping = p.prof && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0;
+    auto stamp = [&](int s, int i) {
+      if (stamping) p.prof[(size_t)s * 8 + i] = gtimer();
+    };
+
+    // One recurrent product, number k = 0, 1, ...: wait for the MMAs, exchange inside the group.
+    // acc[g][j] receives the sum of this thread's unit (forward: gate g) for batch entry b0 + j.
+    // `good` falls when one of this thread's waits has run out; the steps are gone through to the end all the same.
+    bool good = true;
+    auto product = [&](int k, int s, float (*acc)[3]) {
+      const uint32_t tag = (uint32_t)k + 1, parity = (uint32_t)k & 1;
+      if (good && !mbar_wait(done_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutMma);
       stamp(s, 1);
-      if (!mbar_wait(done_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutMma);
-      good = __all_sync(0xffffffffu, good) != 0;
+      if (__all_sync(0xffffffffu, good)) send(tag, parity);
+      else good = false;
+      sent_sync();
       stamp(s, 2);
-      tc_fence_after();
-      if (good) {
-        uint32_t v[NB + 2];
-        v[NB] = v[NB + 1] = 0;
-        tc_ld<NB>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(tile * NB), v);
-        if (row_ok) {
-          if (owner == q) {
-#pragma unroll
-            for (int k = 0; k < kPacks; k++)
-              if (k >= pk_lo && k < pk_hi)
-#pragma unroll
-                for (int j = 0; j < 3; j++)
-                  if (3 * k + j < NB) own_s[rr * kOwnStride + 3 * k + j] = __uint_as_float(v[3 * k + j]);
-          } else {
-            uint4* o = xout + (size_t)parity * xslot;
-#pragma unroll
-            for (int k = 0; k < kPacks; k++)
-              if (k >= pk_lo && k < pk_hi) st_pack(o + k * kRows, make_uint4(v[3 * k], v[3 * k + 1], v[3 * k + 2], tag));
-          }
-        }
-      }
-      if (!workers_sync_and(good)) return false;
-      stamp(s, 3);
       if (mine > 0) {
-#pragma unroll
-        for (int g = 0; g < kGates; g++)
-#pragma unroll
-          for (int j = 0; j < 3; j++) acc[g][j] = j < mine ? own_s[(g * kUnits + u) * kOwnStride + b0 + j] : 0.f;
+        uint4 v[C > 1 ? C - 1 : 1][kGates];
+        const uint4* in = xmine + (parity ? xslot : 0);
         if (C > 1) {
-          const uint4* in = xin + (size_t)parity * xslot + pk * kRows + u;
-          // peers one after the other: member q + 1, q + 2, ... of the group
-          uint4 v[C > 1 ? C - 1 : 1][kGates];
 #pragma unroll
           for (int i = 0; i < C - 1; i++)
 #pragma unroll
-            for (int g = 0; g < kGates; g++) v[i][g] = ld_pack(in + (size_t)(i < q ? i : i + 1) * 2 * xslot + g * kUnits);
+            for (int g = 0; g < kGates; g++) v[i][g] = ld_pack(in + (i < q ? i : i + 1) * 2 * xslot + g * kUnits);
+        }
+#pragma unroll
+        for (int g = 0; g < kGates; g++) {
+          const uint4 o = own_mine[g * kUnits];
+          acc[g][0] = __uint_as_float(o.x);
+          acc[g][1] = __uint_as_float(o.y);
+          acc[g][2] = __uint_as_float(o.z);
+        }
+        if (C > 1) {
           uint32_t spins = 0;
           unsigned long long t0 = 0;
           for (;;) {
@@ -632,7 +653,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
               for (int g = 0; g < kGates; g++)
                 if (v[i][g].w != tag) {
                   missing = true;
-                  v[i][g] = ld_pack(in + (size_t)(i < q ? i : i + 1) * 2 * xslot + g * kUnits);
+                  v[i][g] = ld_pack(in + (i < q ? i : i + 1) * 2 * xslot + g * kUnits);
                 }
             if (!missing || !good) break;
             if (((++spins) & 63) == 0) {
@@ -652,106 +673,138 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
             }
         }
       }
-      stamp(s, 4);
-      return true;
+      stamp(s, 3);
+    };
+    // This block's words of a step are on their way: its loaders may begin to poll the others'.
+    auto published = [&] {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(pub_bar);
     };
 
-    bool fine = true;    // this thread's waits; a step ends for all workers when one of them has given up
     if (!BWD) {
       const float bias_r = p.b_hh[dir][u0 + u], bias_z = p.b_hh[dir][H + u0 + u], bias_n = p.b_hh[dir][2 * H + u0 + u];
+      // Running pointers: one step of time further per step of the loop, backwards for direction 1.
+      const ptrdiff_t step = dir ? -1 : 1;
+      const int t_first = dir ? T - 1 : 0;
+      const int gx_row = ND * 3 * H, y_row = ND * H;
+      const float* gx_p = p.gx + ((size_t)t_first * B + b0) * gx_row + dir * 3 * H + u0 + u;
+      float* y_p = p.y + ((size_t)t_first * B + b0) * y_row + dir * H + u0 + u;
+      float4* rsv_p = p.rsv ? p.rsv + ((size_t)(dir * T + t_first) * B + b0) * H + u0 + u : nullptr;
+      uint32_t* ring_p = ring + ring_at(0, u, b0);
       float gx[3][3];
-      auto load_gx = [&](int t) {
+      auto load_gx = [&]() {
 #pragma unroll
         for (int j = 0; j < 3; j++)
           if (j < mine) {
-            const float* g = p.gx + (((size_t)t * B + b0 + j) * ND + dir) * 3 * H + u0 + u;
+            const float* g = gx_p + j * gx_row;
             gx[0][j] = __ldg(g); gx[1][j] = __ldg(g + H); gx[2][j] = __ldg(g + 2 * H);
           }
+        gx_p += step * B * gx_row;
       };
-      load_gx(dir ? T - 1 : 0);
+      load_gx();
       for (int s = 0; s < T; s++) {
-        const int t = dir ? T - 1 - s : s;
         float acc[3][3] = {};
         stamp(s, 0);
-        if (s > 0 && !product((uint32_t)s, s, acc, fine)) break;
+        if (s > 0) product(s - 1, s, acc);
         float4 keep[3];
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-          if (j < mine) {
-            const float hn = bias_n + acc[2][j];
-            const float r_ = sigmoidf_(gx[0][j] + (bias_r + acc[0][j]));
-            const float z = sigmoidf_(gx[1][j] + (bias_z + acc[1][j]));
-            const float n = tanhf(gx[2][j] + r_ * hn);
-            carry[j] = n + z * (carry[j] - n);
-            keep[j] = make_float4(r_, z, n, hn);
-          }
+          const float hn = bias_n + acc[2][j];
+          const float r_ = sigmoidf_(gx[0][j] + (bias_r + acc[0][j]));
+          const float z = sigmoidf_(gx[1][j] + (bias_z + acc[1][j]));
+          const float n = tanhf_(gx[2][j] + r_ * hn);
+          carry[j] = n + z * (carry[j] - n);
+          keep[j] = make_float4(r_, z, n, hn);
         }
         if (s + 1 < T) {
-          uint32_t* o = ring + (size_t)(s & 1) * ring_slot;
+          uint32_t* o = ring_p + ((s & 1) ? ring_slot : 0u);
 #pragma unroll
           for (int j = 0; j < 3; j++)
-            if (j < mine) st_word(o + ring_at(0, u, b0 + j), tagged(carry[j], (uint32_t)s + 1));
+            if (j < mine) st_word(o + j * kKTile, tagged(carry[j], (uint32_t)s + 1));
+          published();
         }
-        stamp(s, 5);
+        stamp(s, 4);
         // The peers do not wait for what follows.
 #pragma unroll
         for (int j = 0; j < 3; j++)
           if (j < mine) {
-            p.y[((size_t)t * B + b0 + j) * (ND * H) + dir * H + u0 + u] = carry[j];
-            if (p.rsv) p.rsv[((size_t)(dir * T + t) * B + b0 + j) * H + u0 + u] = keep[j];
+            y_p[j * y_row] = carry[j];
+            if (rsv_p) rsv_p[j * H] = keep[j];
           }
-        if (s + 1 < T) load_gx(dir ? T - 2 - s : s + 1);
+        y_p += step * B * y_row;
+        if (rsv_p) rsv_p += step * B * H;
+        if (s + 1 < T) load_gx();
       }
     } else {
-      BwdInputs in;
+      const ptrdiff_t step = dir ? 1 : -1;
+      const int t_first = dir ? 0 : T - 1;
+      const int y_row = ND * H, dg_row = ND * 4 * H;
+      const float4* rsv_p = p.rsv + ((size_t)(dir * T + t_first) * B + b0) * H + u0 + u;
+      const float* dy_p = p.dy + ((size_t)t_first * B + b0) * y_row + dir * H + u0 + u;
+      const float* hp_p = p.y + ((ptrdiff_t)t_first + step) * B * y_row + (ptrdiff_t)b0 * y_row + dir * H + u0 + u;   // h of the step before in the forward pass
+      float* dg_p = p.dg + ((size_t)t_first * B + b0) * dg_row + dir * 3 * H + u0 + u;
+      const int dnr_off = (ND * 3 - dir * 2) * H;       // from (dir * 3) * H to (ND * 3 + dir) * H
+      uint32_t* ring_p[3] = {ring + ring_at(0, u, b0), ring + ring_at(1, u, b0), ring + ring_at(2, u, b0)};
+      float4 in_a[3];                                   // r, z, n, W_hn h + b_hn
+      float in_hp[3] = {0.f, 0.f, 0.f}, in_dy[3];
+      auto load_inputs = [&](bool has_prev) {
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+          if (j < mine) {
+            in_a[j] = __ldg(rsv_p + j * H);
+            in_dy[j] = __ldg(dy_p + j * y_row);
+            in_hp[j] = has_prev ? __ldg(hp_p + j * y_row) : 0.f;
+          }
+        rsv_p += step * B * H;
+        dy_p += step * B * y_row;
+        hp_p += step * B * y_row;
+      };
       float sum[4] = {0.f, 0.f, 0.f, 0.f}, part[4] = {0.f, 0.f, 0.f, 0.f};   // bias gradients, in runs of 16 steps
-      load_bwd_inputs(p, in, dir ? 0 : T - 1, dir, u0 + u, b0, mine);
+      load_inputs(T > 1);
       for (int s = 0; s < T; s++) {
-        const int t = dir ? s : T - 1 - s;
         float keep[3], g[4][3];
         stamp(s, 0);
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-          keep[j] = 0.f;
-          if (j < mine) {
-            const float r_ = in.a[j].x, z = in.a[j].y, n = in.a[j].z, hn = in.a[j].w;
-            const float dh = in.dy[j] + carry[j];
-            const float dn = dh * (1.f - z) * (1.f - n * n);
-            g[0][j] = dn * hn * r_ * (1.f - r_);
-            g[1][j] = dh * (in.hp[j] - n) * z * (1.f - z);
-            g[2][j] = dn;
-            g[3][j] = dn * r_;
-            keep[j] = dh * z;
-          }
+          const float r_ = in_a[j].x, z = in_a[j].y, n = in_a[j].z, hn = in_a[j].w;
+          const float dh = in_dy[j] + carry[j];
+          const float dn = dh * (1.f - z) * (1.f - n * n);
+          g[0][j] = dn * hn * r_ * (1.f - r_);
+          g[1][j] = dh * (in_hp[j] - n) * z * (1.f - z);
+          g[2][j] = dn;
+          g[3][j] = dn * r_;
+          keep[j] = dh * z;
         }
         if (s + 1 < T) {
-          uint32_t* o = ring + (size_t)(s & 1) * ring_slot;
+          const uint32_t slot = (s & 1) ? ring_slot : 0u;
 #pragma unroll
           for (int k = 0; k < 3; k++)
 #pragma unroll
             for (int j = 0; j < 3; j++)
-              if (j < mine) st_word(o + ring_at(k, u, b0 + j), tagged(g[k == 2 ? 3 : k][j], (uint32_t)s + 1));
+              if (j < mine) st_word(ring_p[k] + slot + j * kKTile, tagged(g[k == 2 ? 3 : k][j], (uint32_t)s + 1));
+          published();
         }
-        stamp(s, 5);
+        stamp(s, 4);
         // The peers do not wait for what follows.
 #pragma unroll
         for (int j = 0; j < 3; j++)
           if (j < mine) {
-            float* o = p.dg + ((size_t)t * B + b0 + j) * (ND * 4 * H) + u0 + u;
+            float* o = dg_p + j * dg_row;
 #pragma unroll
-            for (int k = 0; k < 3; k++) o[(dir * 3 + k) * H] = g[k][j];
-            o[(ND * 3 + dir) * H] = g[3][j];
+            for (int k = 0; k < 3; k++) o[k * H] = g[k][j];
+            o[dnr_off] = g[3][j];
 #pragma unroll
             for (int k = 0; k < 4; k++) part[k] += g[k][j];
           }
+        dg_p += step * B * dg_row;
         if ((s & 15) == 15) {
 #pragma unroll
           for (int k = 0; k < 4; k++) { sum[k] += part[k]; part[k] = 0.f; }
         }
         if (s + 1 < T) {
-          load_bwd_inputs(p, in, dir ? s + 1 : T - 2 - s, dir, u0 + u, b0, mine);
+          load_inputs(s + 2 < T);
           float acc[1][3] = {};
-          if (!product((uint32_t)s + 1, s, acc, fine)) break;
+          product(s, s, acc);
 #pragma unroll
           for (int j = 0; j < 3; j++) carry[j] = keep[j] + acc[0][j];
         }
@@ -761,21 +814,21 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       if (mine > 0)
 #pragma unroll
         for (int k = 0; k < 4; k++) red[(pk * 4 + k) * kUnits + u] = sum[k] + part[k];
-      workers_sync_and(true);
+      gates_sync();
       if (tid < 4 * kUnits) {
         float v = 0.f;
         for (int i = 0; i < npacks; i++) v += red[i * 4 * kUnits + tid];
         const int k = tid / kUnits;
         float* o = p.db + dir * 6 * H + u0 + tid % kUnits;
-        if (k != 3) o[k * H] = v;               // dr, dz, dn
-        if (k != 2) o[(k == 3 ? 5 : k + 3) * H] = v;   // dr, dz, dn * r
+        if (k != 3) o[k * H] = v;                        // dr, dz, dn
+        if (k != 2) o[(k == 3 ? 5 : k + 3) * H] = v;     // dr, dz, dn * r
       }
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == kWorkers / 32)
+  if (warp == kThreads / 32 - 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTmemCols) : "memory");
 }
 
@@ -789,11 +842,23 @@ bool dims_ok(const GruDims& d) {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-int mma_n(const GruDims& d) { return d.B <= 16 ? 16 : 32; }
-
+// Blocks per group. Fewer blocks: more operand words to poll per block and longer MMA chains; more blocks: more partial
+// sums, and with one block per group no exchange at all. Microseconds per step (B200, both directions; B = 32 | B = 8):
+//   forward   H   128          256          384          512          768          1024
+//     C = 1       1.83 | 1.56  2.28 | 1.77  2.79 | 2.07  3.43 | 2.26  4.49 | 2.91   -   | 3.57
+//     C = 2       2.09 | 1.79  2.29 | 1.84  2.64 | 2.27  2.97 | 2.35  3.37 | 2.62  4.06 | 2.93
+//     C = 4       3.39 | 2.90  3.56 | 3.04  3.62 | 2.96  3.97 | 3.12  4.29 | 3.15  4.58 | 3.44
+//   backward
+//     C = 2       2.66 | 2.07  3.78 | 2.41  4.35 | 3.32  5.07 | 4.00   -   |  -     -   |  -
+//     C = 4       2.51 | 2.03  2.89 | 2.45  3.24 | 2.65  3.65 | 2.85  4.39 | 3.59  5.24 | 4.17
+//     C = 8       2.67 | 2.16  3.00 | 2.42  3.55 | 2.54  3.75 | 2.66  4.09 | 2.86  4.54 | 3.10
+//     C = 16       -   |  -    4.35 | 3.48   -   |  -    5.28 | 3.60  5.49 | 3.92  5.56 | 4.04
+// (Both passes took 7.7 us per step at T = 75, B = 3, H = 512 and 9.3 at B = 32, H = 1024 when blocks exchanged through
+// counters and TMA and all weights lay in shared memory.)
 int choose_split(const GruDims& d, bool bwd) {
-  if (const char* e = getenv(bwd ? "GRU_CB" : "GRU_CF")) return atoi(e);
-  return bwd ? 8 : 4;
+  const bool small = d.B <= 16;
+  if (bwd) return d.H <= (small ? 256 : 512) ? 4 : 8;
+  return d.H <= (small ? 512 : 256) ? 1 : 2;
 }
 
 // Bytes of partial sums (fp32, 32 batch rows, a block's own included) that a step exchanges with the
@@ -815,7 +880,7 @@ cudaError_t launch_as(const Params& p, cudaStream_t stream) {
   auto kernel = gru_persistent_kernel<BWD, C, NB>;
   const int smem = std::max(pl.smem(), kMinSmem);
   dim3 grid(d.H / kUnits, d.ndir), block(kThreads);
-  if (grid.x > (unsigned)kMaxBlocksPerDir || grid.x % C != 0 || pl.ntile > 4 * kMaxGroups) return cudaErrorInvalidValue;
+  if (grid.x > (unsigned)kMaxBlocksPerDir || grid.x % C != 0 || (pl.ntile + 64 / NB - 1) / (64 / NB) > kLoadsPerGroup * kMaxGroups) return cudaErrorInvalidValue;
   // The attribute belongs to a device: set once for each, to all that a block can have.
   static std::atomic<uint64_t> granted{0};
   int dev = 0;
@@ -829,18 +894,6 @@ cudaError_t launch_as(const Params& p, cudaStream_t stream) {
   return cudaLaunchCooperativeKernel((const void*)kernel, grid, block, args, (size_t)smem, stream);
 }
 
-template <bool BWD, int NB>
-cudaError_t launch_split(int c, const Params& p, cudaStream_t stream) {
-  switch (c) {
-    case 1: return launch_as<BWD, 1, NB>(p, stream);
-    case 2: return launch_as<BWD, 2, NB>(p, stream);
-    case 4: return launch_as<BWD, 4, NB>(p, stream);
-    case 8: if (BWD) return launch_as<BWD, BWD ? 8 : 1, NB>(p, stream); break;
-    case 16: if (BWD) return launch_as<BWD, BWD ? 16 : 1, NB>(p, stream); break;
-  }
-  return cudaErrorInvalidValue;
-}
-
 template <bool BWD>
 cudaError_t launch(Params& p, void* scratch, double timeout_s, cudaStream_t stream) {
   char* w = (char*)scratch;
@@ -849,8 +902,10 @@ cudaError_t launch(Params& p, void* scratch, double timeout_s, cudaStream_t stre
   p.xchg = (uint4*)(w + kSyncBytes + ring_bytes(p.d));
   p.timeout_ns = (unsigned long long)(timeout_s * 1e9);
   p.prof = g_prof;
-  const int c = choose_split(p.d, BWD);
-  return mma_n(p.d) == 16 ? launch_split<BWD, 16>(c, p, stream) : launch_split<BWD, 32>(c, p, stream);
+  const bool wide = choose_split(p.d, BWD) > (BWD ? 4 : 1);
+  constexpr int lo = BWD ? 4 : 1, hi = BWD ? 8 : 2;
+  if (p.d.B <= 16) return wide ? launch_as<BWD, hi, 16>(p, stream) : launch_as<BWD, lo, 16>(p, stream);
+  return wide ? launch_as<BWD, hi, 32>(p, stream) : launch_as<BWD, lo, 32>(p, stream);
 }
 
 }  // namespace
