@@ -164,7 +164,7 @@ int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const flo
                     const float* dy, float* dg, float* db, void* scratch, unsigned* status, double timeout_s, void* stream);
 
 /* Training-mode batch normalisation of [N, C, HW] fp32 activations fused with the clipped ReLU behind it
- * (y = clamp(bn(x), 0, clip_hi)); csrc/cuda/bn_clip.h. `acc` = scratch of 2 * C doubles; running_* may be NULL.
+ * (y = clamp(bn(x), 0, clip_hi)); csrc/cuda/bn_clip.h. `acc` = scratch of 2 * (C + 1024) doubles; running_* may be NULL.
  * These need no initialised group. */
 int bc_bn_clip_forward(const float* x, float* y, const float* gamma, const float* beta, float* running_mean, float* running_var,
                        float* save_mean, float* save_rstd, double* acc, int N, int C, int HW, float eps, float momentum, float clip_hi,

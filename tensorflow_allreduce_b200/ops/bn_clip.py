@@ -34,7 +34,7 @@ class _BNClip(torch.autograd.Function):
         y = torch.empty_like(x)
         save_mean = torch.empty(c, dtype=torch.float32, device=x.device)
         save_rstd = torch.empty(c, dtype=torch.float32, device=x.device)
-        acc = torch.empty(2 * c, dtype=torch.float64, device=x.device)
+        acc = torch.empty(2 * (c + 1024), dtype=torch.float64, device=x.device)
         rc = _lib.lib().bc_bn_clip_forward(_ptr(x), _ptr(y), _ptr(weight), _ptr(bias), _ptr(running_mean), _ptr(running_var),
                                            _ptr(save_mean), _ptr(save_rstd), _ptr(acc), n, c, hw, float(eps), float(momentum),
                                            float(clip), C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream))
@@ -54,7 +54,7 @@ class _BNClip(torch.autograd.Function):
         dx = torch.empty_like(x)
         dw = torch.empty_like(weight)
         db = torch.empty_like(bias)
-        acc = torch.empty(2 * c, dtype=torch.float64, device=x.device)
+        acc = torch.empty(2 * (c + 1024), dtype=torch.float64, device=x.device)
         rc = _lib.lib().bc_bn_clip_backward(_ptr(x), _ptr(dy), _ptr(weight), _ptr(bias), _ptr(save_mean), _ptr(save_rstd), _ptr(dx),
                                             _ptr(dw), _ptr(db), _ptr(acc), n, c, hw, ctx.clip,
                                             C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream))
