@@ -31,6 +31,7 @@ class BuildNative(Command):
         from tensorflow_allreduce_b200 import build
 
         print(build.build())
+        print(build.build_ext())
         if self.debug_kernels:
             print(build.build(debug=True))
 

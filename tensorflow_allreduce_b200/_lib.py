@@ -107,7 +107,7 @@ def _declare(lib):
         "bc_gru_scratch_bytes": (ll, [i, i, i, i]),
         "bc_gru_forward": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
         "bc_gru_backward": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
-        "bc_bn_clip_forward": (i, [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, f, f, vp]),
+        "bc_bn_clip_forward": (i, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, f, f, vp]),
         "bc_bn_clip_backward": (i, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, vp]),
         "bc_test_validate": (i, [i, P(i), P(i), P(i), P(i), P(ll), cp, i, P(ll)]),
     }
@@ -148,6 +148,42 @@ def lib():
         _declare(loaded)
         _lib = loaded
     return _lib
+
+
+_ext = None
+
+
+def ext():
+    """The extension module over torch's C++ API (`csrc/torch/bindings.cc`), built first if needed. The native library is
+    loaded before it, because the extension takes its symbols from there."""
+    global _ext
+    if _ext is not None:
+        return _ext
+    lib()
+    with _lock:
+        if _ext is not None:
+            return _ext
+        import importlib.machinery
+        import importlib.util
+
+        from . import build as _build
+
+        if os.environ.get("BC_NO_BUILD", "0") != "1" and _build.needs_build_ext():
+            import fcntl
+
+            with open(_build.LIBDIR / ".build.lock", "w") as lk:
+                fcntl.flock(lk, fcntl.LOCK_EX)
+                try:
+                    _build.build_ext()
+                finally:
+                    fcntl.flock(lk, fcntl.LOCK_UN)
+        if not _build.EXT.exists():
+            raise NativeError(f"native extension missing: {_build.EXT}")
+        loader = importlib.machinery.ExtensionFileLoader("bcoll_torch", str(_build.EXT))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("bcoll_torch", loader))
+        loader.exec_module(module)
+        _ext = module
+    return _ext
 
 
 def last_error() -> str:

@@ -23,6 +23,7 @@ LIBDIR = PKG / "lib"
 OBJDIR = LIBDIR / "obj"
 LIB = LIBDIR / "libbcoll.so"
 LIB_DEBUG = LIBDIR / "libbcoll_debug.so"   # same sources with -DBC_DEBUG: bounds-checked kernels
+EXT = LIBDIR / "bcoll_torch.so"            # native call paths over torch's C++ API (csrc/torch), loaded beside either of them
 
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.environ.get("NVCC", str(Path(CUDA_HOME) / "bin" / "nvcc"))
@@ -34,7 +35,7 @@ CXX_FLAGS = ["-O2", "-g1", "-fPIC", "-std=c++17", "-Wall", "-pthread", f"-I{CUDA
 
 
 def _sources():
-    cc = sorted(p for p in CSRC.rglob("*.cc") if "selftest" not in p.parts)
+    cc = sorted(p for p in CSRC.rglob("*.cc") if "selftest" not in p.parts and "torch" not in p.relative_to(CSRC).parts)
     cu = sorted(p for p in CSRC.rglob("*.cu"))
     return cc, cu
 
@@ -132,6 +133,49 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False, 
     return LIB
 
 
+def _ext_fingerprint() -> str:
+    import hashlib
+
+    import torch
+
+    h = hashlib.sha256(f"{torch.__version__} {sys.version} {CXX_FLAGS}".encode())
+    for p in (CSRC / "torch" / "bindings.cc", CSRC / "bcoll.h"):
+        h.update(p.read_bytes())
+    return h.hexdigest()
+
+
+def needs_build_ext() -> bool:
+    stamp = LIBDIR / ".fingerprint_torch"
+    return not EXT.exists() or not stamp.exists() or stamp.read_text().strip() != _ext_fingerprint()
+
+
+def build_ext(force: bool = False, verbose: bool = False) -> Path:
+    """Compile `csrc/torch/bindings.cc` against the installed torch into `lib/bcoll_torch.so`. It takes the native library's
+    symbols from whichever variant the process has loaded."""
+    if not force and not needs_build_ext():
+        return EXT
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    LIBDIR.mkdir(parents=True, exist_ok=True)
+    tmp = EXT.with_suffix(".so.tmp")
+    inc = [f"-I{p}" for p in cpp_extension.include_paths()] + [f"-I{sysconfig.get_paths()['include']}", f"-I{CUDA_HOME}/include"]
+    cmd = [CXX, "-O2", "-fPIC", "-std=c++17", "-pthread", "-shared", "-DTORCH_EXTENSION_NAME=bcoll_torch", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + inc + [
+        str(CSRC / "torch" / "bindings.cc"), "-o", str(tmp), f"-L{Path(torch.__file__).parent / 'lib'}",
+        "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"compiling the torch bindings failed:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, EXT)
+    (LIBDIR / ".fingerprint_torch").write_text(_ext_fingerprint() + "\n")
+    return EXT
+
+
 def _sanitizer_cxx(sanitizer: str) -> str:
     """First C++ compiler that can link a program with -fsanitize=<sanitizer> (a toolchain may
     ship without the sanitizer run-time libraries)."""
@@ -194,3 +238,4 @@ if __name__ == "__main__":
     ap.add_argument("--debug", action="store_true", help="build the bounds-checked variant (-DBC_DEBUG, lib/libbcoll_debug.so)")
     a = ap.parse_args()
     print(build(force=a.force, verbose=a.verbose, ptxas_info=a.ptxas, debug=a.debug))
+    print(build_ext(force=a.force, verbose=a.verbose))

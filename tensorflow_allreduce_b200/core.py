@@ -40,7 +40,7 @@ _DTYPES = {
     torch.float64: 5, torch.uint8: 6,
 }
 
-_state = {"config": None, "device": None}
+_state = {"config": None, "device": None, "alone": False}   # alone: a GPU group of one rank
 _counter_lock = threading.Lock()
 _counters = {"allreduce": itertools.count(), "allgather": itertools.count(), "blob": itertools.count(),
              "broadcast": itertools.count(), "barrier": itertools.count()}
@@ -139,6 +139,7 @@ def init(device=None, config: Optional[Config] = None, rank: Optional[int] = Non
                       cfg.nvls_min_kb << 10, int(cfg.nvls), cfg.max_blocks, cfg.symm_code, cfg.fault.encode()), "bc_init")
     _state["config"] = cfg
     _state["device"] = dev_index
+    _state["alone"] = dev_index >= 0 and size_ == 1
     if dev_index >= 0 and cfg.overlap_blocks > 0:
         _call(lib.bc_set_option(b"overlap_blocks", cfg.overlap_blocks), "bc_set_option")
     if dev_index >= 0:
@@ -163,6 +164,7 @@ def shutdown() -> None:
         _call(lib.bc_shutdown(), "bc_shutdown")
     _state["config"] = None
     _state["device"] = None
+    _state["alone"] = False
 
 
 def _dump_stats_jsonl() -> None:
@@ -393,6 +395,12 @@ def allreduce(tensor: torch.Tensor, average: Optional[bool] = None, name: Option
         if average:
             g_vals = g_vals / size() if g_vals.is_floating_point() else torch.div(g_vals, size(), rounding_mode="trunc")
         return torch.sparse_coo_tensor(g_idx.t(), g_vals, t.shape)
+    if tensor.is_cuda and _state["alone"]:
+        # a group of one rank: nobody to ask, no private stream to order with
+        red, average = _resolve_reduction(op, average)
+        out = _lib.ext().allreduce_alone(name or _auto_name("allreduce"), tensor, average, red)
+        if out is not None:
+            return out
     return allreduce_async(tensor, average=average, name=name, op=op).wait()
 
 

@@ -62,6 +62,10 @@ typedef void* (*bc_alloc_fn)(long long handle, long long total_rows, void* user,
 long long bc_allreduce_async(const char* name, const void* in, void* out, int dtype, int ndim, const long long* shape,
                              int device_kind, int average, int zero_copy, void* ready_event, int reduce_op);
 /* reduce_op: 0 sum, 1 prod, 2 min, 3 max (averaging goes with the sum only). */
+/* The same reduction in a group of one rank, on the caller's stream and at once: nobody has to be asked. Returns 1 when it
+ * was launched, 0 when the call has to be negotiated (more than one rank, no GPU, a fault armed, device timing on). */
+int bc_allreduce_alone(const char* name, const void* in, void* out, int dtype, long long count, int device, int average, int reduce_op,
+                       void* stream);
 long long bc_allgather_async(const char* name, const void* in, int dtype, int ndim, const long long* shape, int device_kind,
                              bc_alloc_fn alloc, void* user, void* ready_event);
 int bc_wait(long long handle, double timeout_s);
@@ -164,11 +168,11 @@ int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const flo
                     const float* dy, float* dg, float* db, void* scratch, unsigned* status, double timeout_s, void* stream);
 
 /* Training-mode batch normalisation of [N, C, HW] fp32 activations fused with the clipped ReLU behind it
- * (y = clamp(bn(x), 0, clip_hi)); csrc/cuda/bn_clip.h. `acc` = scratch of 2 * (C + 1024) doubles; running_* may be NULL.
+ * (y = clamp(bn(x), 0, clip_hi)); csrc/cuda/bn_clip.h. `acc` = scratch of 2 * (C + 1024) doubles; running_* and `batches` (a counter that goes up by one) may be NULL.
  * These need no initialised group. */
 int bc_bn_clip_forward(const float* x, float* y, const float* gamma, const float* beta, float* running_mean, float* running_var,
-                       float* save_mean, float* save_rstd, double* acc, int N, int C, int HW, float eps, float momentum, float clip_hi,
-                       void* stream);
+                       long long* batches, float* save_mean, float* save_rstd, double* acc, int N, int C, int HW, float eps, float momentum,
+                       float clip_hi, void* stream);
 int bc_bn_clip_backward(const float* x, const float* dy, const float* gamma, const float* beta, const float* save_mean,
                         const float* save_rstd, float* dx, float* dgamma, float* dbeta, double* acc, int N, int C, int HW,
                         float clip_hi, void* stream);

@@ -228,6 +228,15 @@ long long bc_allgather_async(const char* name, const void* in, int dtype, int nd
   API_END(-1)
 }
 
+int bc_allreduce_alone(const char* name, const void* in, void* out, int dtype, long long count, int device, int average, int reduce_op,
+                       void* stream) {
+  API_BEGIN
+  if (reduce_op < 0 || reduce_op > (int)ReduceOp::MAX) throw Error("allreduce: unknown reduction");
+  if (average && reduce_op != (int)ReduceOp::SUM) throw Error("allreduce: averaging goes with the sum only");
+  return rt().allreduce_alone(name, in, out, (size_t)count, (DType)dtype, device, stream) ? 1 : 0;
+  API_END(-1)
+}
+
 int bc_wait(long long handle, double timeout_s) {
   API_BEGIN
   rt().wait(handle, timeout_s);
@@ -569,10 +578,10 @@ int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const flo
 // ---- batch normalisation fused with the clipped ReLU ---------------------------------------------
 
 int bc_bn_clip_forward(const float* x, float* y, const float* gamma, const float* beta, float* running_mean, float* running_var,
-                       float* save_mean, float* save_rstd, double* acc, int N, int C, int HW, float eps, float momentum, float clip_hi,
-                       void* stream) {
+                       long long* batches, float* save_mean, float* save_rstd, double* acc, int N, int C, int HW, float eps, float momentum,
+                       float clip_hi, void* stream) {
   API_BEGIN
-  check_cuda(gpu::bn_clip_forward(x, y, gamma, beta, running_mean, running_var, save_mean, save_rstd, acc, N, C, HW, eps, momentum,
+  check_cuda(gpu::bn_clip_forward(x, y, gamma, beta, running_mean, running_var, batches, save_mean, save_rstd, acc, N, C, HW, eps, momentum,
                                   clip_hi, (cudaStream_t)stream), "batch-norm + clip forward launch");
   return 0;
   API_END(-1)

@@ -23,6 +23,7 @@
 #include "collectives.h"
 #include "device_prims.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace bc {
@@ -452,10 +453,29 @@ __global__ void __launch_bounds__(512, 2) allreduce_kernel(const __grid_constant
   }
 }
 
-__global__ void __launch_bounds__(512) copy_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, size_t npacks,
-                                                    char* dtail, const char* stail, int ntail) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < npacks; i += stride) dst[i] = src[i];
+// Plain copy, bound by HBM (small ones by latency): U 16-byte loads in flight per thread, a block takes runs of U x 8 KB.
+constexpr int kCopyThreads = 512;
+template <int kCopyUnroll>
+__global__ void __launch_bounds__(kCopyThreads) copy_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, size_t npacks,
+                                                            char* dtail, const char* stail, int ntail) {
+  constexpr size_t kRun = (size_t)kCopyThreads * kCopyUnroll;
+  for (size_t base = blockIdx.x * kRun; base < npacks; base += gridDim.x * kRun) {
+    uint4 v[kCopyUnroll];
+    const size_t i = base + threadIdx.x;
+    if (base + kRun <= npacks) {
+#pragma unroll
+      for (int u = 0; u < kCopyUnroll; u++) v[u] = __ldcs(src + i + u * kCopyThreads);
+#pragma unroll
+      for (int u = 0; u < kCopyUnroll; u++) __stcs(dst + i + u * kCopyThreads, v[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < kCopyUnroll; u++)
+        if (i + u * kCopyThreads < npacks) v[u] = __ldcs(src + i + u * kCopyThreads);
+#pragma unroll
+      for (int u = 0; u < kCopyUnroll; u++)
+        if (i + u * kCopyThreads < npacks) __stcs(dst + i + u * kCopyThreads, v[u]);
+    }
+  }
   if (blockIdx.x == 0 && (int)threadIdx.x < ntail) dtail[threadIdx.x] = stail[threadIdx.x];
 }
 
@@ -535,10 +555,14 @@ cudaError_t launch_copy(void* dst, const void* src, size_t bytes, cudaStream_t s
   if ((((uintptr_t)dst | (uintptr_t)src) & 15) != 0) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s);
   const size_t npacks = bytes / 16;
   const int ntail = (int)(bytes % 16);
-  int blocks = (int)((npacks + 512 * 8 - 1) / (512 * 8));
-  if (blocks < 1) blocks = 1;
-  if (blocks > 592) blocks = 592;
-  copy_kernel<<<blocks, 512, 0, s>>>((uint4*)dst, (const uint4*)src, npacks, (char*)dst + npacks * 16,
+  // One load per thread while all of them are in flight at once anyway (592 blocks are four per SM), so that a small tensor
+  // is spread over as many SMs as it has blocks; eight for tensors of several passes.
+  const size_t kOnePass = 592u * kCopyThreads;
+  const int unroll = npacks <= kOnePass ? 1 : npacks <= 4 * kOnePass ? 4 : 8;
+  const size_t run = (size_t)kCopyThreads * unroll;
+  const int blocks = (int)std::max<size_t>(1, std::min<size_t>((npacks + run - 1) / run, 592));
+  auto kernel = unroll == 1 ? copy_kernel<1> : unroll == 4 ? copy_kernel<4> : copy_kernel<8>;
+  kernel<<<blocks, kCopyThreads, 0, s>>>((uint4*)dst, (const uint4*)src, npacks, (char*)dst + npacks * 16,
                                      (const char*)src + npacks * 16, ntail);
   return cudaGetLastError();
 }

@@ -151,7 +151,7 @@ template <bool WARPS, bool VEC>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bn_apply_kernel(const float* __restrict__ x, float* __restrict__ y, const double2* __restrict__ part,
                                                                          const float* __restrict__ gamma, const float* __restrict__ beta,
                                                                          float* __restrict__ save_mean, float* __restrict__ save_rstd,
-                                                                         float* running_mean, float* running_var, int N, int C, int HW, float eps,
+                                                                         float* running_mean, float* running_var, long long* batches, int N, int C, int HW, float eps,
                                                                          float momentum, float clip_hi) {
   cudaGridDependencySynchronize();
   const int c = blockIdx.y;
@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm) bn_apply_kernel(const 
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     save_mean[c] = mean;
     save_rstd[c] = rstd;
+    if (batches && c == 0) *batches += 1;
     if (running_mean) {
       const float unbiased = (float)(var_d * (m / (m > 1.0 ? m - 1.0 : 1.0)));
       running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * mean;
@@ -312,13 +313,13 @@ cudaError_t launch(bool dependent, K kernel, dim3 grid, cudaStream_t stream, A..
 }
 
 template <bool WARPS, bool VEC>
-cudaError_t forward(const float* x, float* y, const float* gamma, const float* beta, float* running_mean, float* running_var, float* save_mean,
+cudaError_t forward(const float* x, float* y, const float* gamma, const float* beta, float* running_mean, float* running_var, long long* batches, float* save_mean,
                     float* save_rstd, double2* part, int N, int C, int HW, float eps, float momentum, float clip_hi, cudaStream_t stream) {
   const dim3 grid(blocks_per_channel(N, C, HW), C);
   cudaError_t e = launch(false, bn_stats_kernel<WARPS, VEC>, grid, stream, x, part, N, C, HW);
   if (e != cudaSuccess) return e;
   return launch(true, bn_apply_kernel<WARPS, VEC>, grid, stream, x, y, (const double2*)part, gamma, beta, save_mean, save_rstd, running_mean,
-                running_var, N, C, HW, eps, momentum, clip_hi);
+                running_var, batches, N, C, HW, eps, momentum, clip_hi);
 }
 
 template <bool WARPS, bool VEC>
@@ -334,12 +335,12 @@ cudaError_t backward(const float* x, const float* dy, const float* gamma, const 
 }  // namespace
 
 cudaError_t bn_clip_forward(const float* x, float* y, const float* gamma, const float* beta, float* running_mean, float* running_var,
-                            float* save_mean, float* save_rstd, double* acc, int N, int C, int HW, float eps, float momentum,
+                            long long* batches, float* save_mean, float* save_rstd, double* acc, int N, int C, int HW, float eps, float momentum,
                             float clip_hi, cudaStream_t stream) {
   if (N <= 0 || C <= 0 || HW <= 0 || C > 65535) return cudaErrorInvalidValue;
   const bool vec = aligned16({x, y}), warps = HW < kShortPlane;
   auto fn = warps ? (vec ? forward<true, true> : forward<true, false>) : (vec ? forward<false, true> : forward<false, false>);
-  return fn(x, y, gamma, beta, running_mean, running_var, save_mean, save_rstd, (double2*)acc, N, C, HW, eps, momentum, clip_hi, stream);
+  return fn(x, y, gamma, beta, running_mean, running_var, batches, save_mean, save_rstd, (double2*)acc, N, C, HW, eps, momentum, clip_hi, stream);
 }
 
 cudaError_t bn_clip_backward(const float* x, const float* dy, const float* gamma, const float* beta, const float* save_mean,

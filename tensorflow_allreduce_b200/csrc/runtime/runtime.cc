@@ -193,6 +193,7 @@ Runtime::~Runtime() {
     shutdown();
   } catch (...) {
   }
+  for (void* e : done_events_) cudaEventDestroy((cudaEvent_t)e);
   if (wake_fd_ >= 0) ::close(wake_fd_);
 }
 
@@ -269,11 +270,16 @@ int64_t Runtime::enqueue(std::unique_ptr<OpRecord> rec_in) {
              "a collective named '" << rec->name << "' is already in flight on this rank");
     if (rec->device == DeviceKind::GPU) {
       BC_CHECK(comm_ != nullptr, "GPU tensor passed, but init() ran without a GPU device");
-      cudaEvent_t ev = nullptr;
-      cudaSetDevice(opt_.device);
-      cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-      BC_CHECK(e == cudaSuccess, "cudaEventCreate: " << cudaGetErrorString(e));
-      rec->done_event = ev;
+      if (!done_events_.empty()) {
+        rec->done_event = done_events_.back();
+        done_events_.pop_back();
+      } else {
+        cudaEvent_t ev = nullptr;
+        cudaSetDevice(opt_.device);
+        cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        BC_CHECK(e == cudaSuccess, "cudaEventCreate: " << cudaGetErrorString(e));
+        rec->done_event = ev;
+      }
     }
     rec->id = next_id_++;
     rec->t_enqueue = now_s();
@@ -326,11 +332,45 @@ void Runtime::release(int64_t handle) {
     if (it == handles_.end()) return;
     rec = it->second;
     handles_.erase(it);
+    // An operation that is still in flight records its event later: that event is not for reuse.
+    if (rec->done_event && rec->state != OpRecord::PENDING && done_events_.size() < kDoneEvents) {
+      done_events_.push_back(rec->done_event);
+      rec->done_event = nullptr;
+    }
   }
   if (rec->done_event) {
     cudaEventDestroy((cudaEvent_t)rec->done_event);
     rec->done_event = nullptr;
   }
+}
+
+bool Runtime::allreduce_alone(const char* name, const void* in, void* out, size_t count, DType dtype, int device, void* stream) {
+  if (t_.size != 1 || !comm_ || device != opt_.device || device_timing()) return false;
+  StatEntry e;
+  e.t_enqueue = now_s();
+  e.name = name;
+  {
+    std::lock_guard<std::mutex> g(mu_);
+    if (broken_.load()) throw CommLost("communicator is broken: " + broken_reason_);
+    BC_CHECK(!stop_.load(), "the runtime has been shut down");
+    BC_CHECK(table_.find(e.name) == table_.end(), "a collective named '" << e.name << "' is already in flight on this rank");
+    if (fault_.kind != FaultSpec::NONE) return false;
+  }
+  BC_CHECK(comm_->device_status() == 0, "an earlier device-side wait timed out (status 0x" << std::hex << comm_->device_status()
+           << "); the communicator cannot be used any more");
+  NvtxRange range("bcoll.allreduce");
+  e.bytes = (int64_t)(count * dtype_size(dtype));
+  cudaError_t rc = in == out ? cudaSuccess : gpu::launch_copy(out, in, (size_t)e.bytes, (cudaStream_t)stream);
+  BC_CHECK(rc == cudaSuccess, "allreduce: " << cudaGetErrorString(rc));
+  e.op = (int)OpType::ALLREDUCE;
+  e.algo = (int)gpu::Algo::ONE_SHOT;
+  e.device = (int)DeviceKind::GPU;
+  e.t_negotiated = e.t_enqueue;      // nobody to ask
+  e.t_done = now_s();
+  std::lock_guard<std::mutex> g(stats_mu_);
+  stats_.push_back(std::move(e));
+  if (stats_.size() > 4096) stats_.pop_front();
+  return true;
 }
 
 std::vector<std::string> Runtime::blob_gather(const std::string& name, const std::string& mine) {

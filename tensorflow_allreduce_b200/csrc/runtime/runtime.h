@@ -142,6 +142,10 @@ class Runtime {
   std::shared_ptr<OpRecord> get(int64_t handle);
   void release(int64_t handle);
 
+  // The reduction of a GPU tensor over a group of one rank: a copy on the caller's stream. False if the call has to be
+  // negotiated.
+  bool allreduce_alone(const char* name, const void* in, void* out, size_t count, DType dtype, int device, void* stream);
+
   // Convenience: host allgather of small blobs through the negotiated path.
   std::vector<std::string> blob_gather(const std::string& name, const std::string& mine);
 
@@ -204,6 +208,8 @@ class Runtime {
   std::deque<std::shared_ptr<OpRecord>> queue_;                       // enqueued, not yet seen by the thread
   std::unordered_map<std::string, std::shared_ptr<OpRecord>> table_;  // in flight, by name
   std::unordered_map<int64_t, std::shared_ptr<OpRecord>> handles_;
+  std::vector<void*> done_events_;                                    // ready for reuse (at most kDoneEvents)
+  static constexpr size_t kDoneEvents = 64;
   int64_t next_id_ = 1;
   std::atomic<bool> broken_{false};
   std::atomic<bool> stop_{false};
