@@ -65,6 +65,60 @@ __device__ __forceinline__ void push_slab(char* dst, const char* src, size_t n, 
   for (size_t i = body + tid; i < n; i += nthreads) dst[i] = src[i];
 }
 
+// 16 bytes from `src`, which is only aligned to W bytes.
+template <int W>
+__device__ __forceinline__ uint4 ld_unaligned16(const char* src) {
+  if constexpr (W == 16) {
+    return *reinterpret_cast<const uint4*>(src);
+  } else if constexpr (W == 8) {
+    const uint2 a = reinterpret_cast<const uint2*>(src)[0], b = reinterpret_cast<const uint2*>(src)[1];
+    return make_uint4(a.x, a.y, b.x, b.y);
+  } else if constexpr (W == 4) {
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(src);
+    return make_uint4(p[0], p[1], p[2], p[3]);
+  } else {
+    const uint16_t* p = reinterpret_cast<const uint16_t*>(src);
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) w[i] = (uint32_t)p[2 * i] | ((uint32_t)p[2 * i + 1] << 16);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// Copy `n` bytes from local `src` to all P destinations, which have the same alignment; the grid as a whole. Every byte of the
+// slab is loaded once and stored P times (pushing the slab to one rank after the other loaded it P times, and with one store
+// per load the small number of blocks that a rank has kept too little in flight: 8 emulated ranks, 33 MB of slabs, 76 us).
+// Stores are 16 bytes wide on aligned addresses whatever the alignment of the source. The order of the ranks is `first`,
+// first + 1, ...: at any moment the P ranks write to P different targets.
+template <int W>
+__device__ __forceinline__ void push_slab_all(char* const* dst, int P, int first, const char* src, size_t n, size_t tid, size_t nthreads) {
+  size_t head = (16 - ((uintptr_t)dst[0] & 15)) & 15;
+  if (head > n) head = n;
+  const size_t k = (n - head) / 16, tail = (n - head) & 15;
+  constexpr int U = 4;
+  auto all = [&](size_t at, uint4 v) {
+    for (int j = 0; j < P; j++) {
+      int p = first + j;
+      if (p >= P) p -= P;
+      st16(dst[p] + at, v);
+    }
+  };
+  size_t i = tid;
+  for (; i + (U - 1) * nthreads < k; i += U * nthreads) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = ld_unaligned16<W>(src + head + (i + u * nthreads) * 16);
+#pragma unroll
+    for (int u = 0; u < U; u++) all(head + (i + u * nthreads) * 16, v[u]);
+  }
+  for (; i < k; i += nthreads) all(head + i * 16, ld_unaligned16<W>(src + head + i * 16));
+  if (tid < head + tail) {
+    const size_t at = tid < head ? tid : head + k * 16 + (tid - head);
+    const char v = src[at];
+    for (int p = 0; p < P; p++) dst[p][at] = v;
+  }
+}
+
 // Multicast variant: `dst` is an address in the multicast mapping, so every store lands in every
 // rank's segment. multimem stores are at least 4 bytes wide; the caller guarantees that dst, src
 // and n are multiples of 4.
@@ -116,6 +170,7 @@ __global__ void __launch_bounds__(512) allgatherv_kernel(const __grid_constant__
   const int P = c.world, me = c.rank;
   __shared__ unsigned long long s_bytes[kMaxRanks];
   __shared__ unsigned long long s_off[kMaxRanks];
+  __shared__ char* s_dst[kMaxRanks];
 
   uint32_t epoch = load_epoch(c);
   // Publish my size and output offset into slot [block][me] of every peer's metadata area.
@@ -160,10 +215,21 @@ __global__ void __launch_bounds__(512) allgatherv_kernel(const __grid_constant__
     push_slab_mc(R.mc_base + s_off[0] + disp, R.in, (size_t)R.bytes, tid, nthreads);
   } else {
     // Start with the next rank so that at any moment the P ranks write to P different targets.
-    for (int k = 0; k < P; k++) {
-      const int p = (me + 1 + k) % P;
-      push_slab(R.base[p] + s_off[p] + disp, R.in, (size_t)R.bytes, tid, nthreads);
-    }
+    const int next = me + 1 < P ? me + 1 : 0;
+    if ((int)threadIdx.x < P) s_dst[threadIdx.x] = R.base[threadIdx.x] + s_off[threadIdx.x] + disp;
+    __syncthreads();
+    bool alike = true;
+    for (int p = 1; p < P; p++) alike = alike && (((uintptr_t)s_dst[p] ^ (uintptr_t)s_dst[0]) & 15) == 0;
+    const unsigned rel = (unsigned)(((uintptr_t)s_dst[0] - (uintptr_t)R.in) & 15);
+    if (alike && rel == 0) push_slab_all<16>(s_dst, P, next, R.in, (size_t)R.bytes, tid, nthreads);
+    else if (alike && rel == 8) push_slab_all<8>(s_dst, P, next, R.in, (size_t)R.bytes, tid, nthreads);
+    else if (alike && (rel & 3) == 0) push_slab_all<4>(s_dst, P, next, R.in, (size_t)R.bytes, tid, nthreads);
+    else if (alike && (rel & 1) == 0) push_slab_all<2>(s_dst, P, next, R.in, (size_t)R.bytes, tid, nthreads);
+    else
+      for (int k = 0; k < P; k++) {
+        const int p = (next + k) % P;
+        push_slab(s_dst[p], R.in, (size_t)R.bytes, tid, nthreads);
+      }
   }
   if (P > 1) peer_barrier(c, epoch);
   store_epoch(c, epoch);
