@@ -86,6 +86,7 @@ def _declare(lib):
         "bc_stream_wait_event": (i, [vp, vp]),
         "bc_allreduce_direct": (i, [i, vp, vp, ll, i, i, vp, vp]),
         "bc_fused_step": (i, [i, vp, ll, i, vp, vp, vp, vp, P(OptHyper), f, vp, vp, i]),
+        "bc_fused_step_alone": (i, [i, vp, vp, ll, i, vp, vp, vp, vp, P(OptHyper)]),
         "bc_set_option": (i, [cp, ll]),
         "bc_set_allreduce_profile": (i, [vp]),
         "bc_allgatherv_direct": (i, [i, vp, ll, vp, ll, vp, vp, vp]),

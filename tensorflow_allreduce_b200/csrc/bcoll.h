@@ -109,6 +109,9 @@ int bc_allreduce_direct(int channel, const void* in, void* out, long long count,
  * persistent compute kernel leaves free (option "overlap_blocks"), so all its blocks can be resident. */
 int bc_fused_step(int channel, void* grad, long long count, int dtype, void* param, float* master, float* s1, float* s2,
                   const bc_opt_hyper* h, float scale, void* wait_event, void* record_event, int beside_compute);
+/* The update in a group of one rank, on the caller's stream (default stream: NULL): nothing to order with peers. */
+int bc_fused_step_alone(int channel, void* stream, void* grad, long long count, int dtype, void* param, float* master, float* s1,
+                        float* s2, const bc_opt_hyper* h);
 /* Run-time switches: "device_timing" (1: ordered launches and negotiated GPU allreduces are bracketed
  * by timing events and their records in bc_stats_json() carry "device_us"), "overlap_blocks". */
 int bc_set_option(const char* key, long long value);

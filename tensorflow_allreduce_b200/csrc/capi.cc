@@ -374,25 +374,40 @@ int bc_allreduce_direct(int channel, const void* in, void* out, long long count,
   API_END(-1)
 }
 
-int bc_fused_step(int channel, void* grad, long long count, int dtype, void* param, float* master, float* s1, float* s2,
-                  const bc_opt_hyper* h, float scale, void* wait_event, void* record_event, int beside_compute) {
-  API_BEGIN
+// `s`: the stream of the launch, a channel's or the caller's.
+static int fused_step_on(cudaStream_t s, int channel, void* grad, long long count, int dtype, void* param, float* master, float* s1, float* s2,
+                         const bc_opt_hyper* h, float scale, void* wait_event, void* record_event, bool beside_compute) {
   NvtxRange range("bcoll.fused_step");
-  require_one_host("the fused update");
-  check_channel(channel);
   gpu::Comm& c = comm();
   require_healthy(c);
-  cudaStream_t s = c.stream(channel);
   stream_prologue(s, wait_event);
   static_assert(sizeof(bc_opt_hyper) == sizeof(gpu::OptHyper), "bc_opt_hyper must mirror OptHyper");
   gpu::OptHyper hh;
   memcpy(&hh, h, sizeof(hh));
   TimedLaunch timed;
   if (rt().device_timing()) timed = rt().timed_begin(s);
-  gpu::Algo a = c.fused_step(channel, grad, (size_t)count, (DType)dtype, param, master, s1, s2, hh, scale, nullptr, beside_compute != 0);
+  gpu::Algo a = c.fused_step(channel, grad, (size_t)count, (DType)dtype, param, master, s1, s2, hh, scale, s, beside_compute);
   if (timed.stop) rt().timed_end(timed, s, "fused_step", (int)a, c.last_blocks, count * (long long)dtype_size((DType)dtype), channel);
   stream_epilogue(s, record_event);
   return (int)a;
+}
+
+int bc_fused_step(int channel, void* grad, long long count, int dtype, void* param, float* master, float* s1, float* s2,
+                  const bc_opt_hyper* h, float scale, void* wait_event, void* record_event, int beside_compute) {
+  API_BEGIN
+  require_one_host("the fused update");
+  check_channel(channel);
+  return fused_step_on(comm().stream(channel), channel, grad, count, dtype, param, master, s1, s2, h, scale, wait_event, record_event,
+                       beside_compute != 0);
+  API_END(-1)
+}
+
+int bc_fused_step_alone(int channel, void* stream, void* grad, long long count, int dtype, void* param, float* master, float* s1, float* s2,
+                        const bc_opt_hyper* h) {
+  API_BEGIN
+  check_channel(channel);
+  if (rt().size() > 1) throw Error("bc_fused_step_alone is for a group of one rank");
+  return fused_step_on((cudaStream_t)stream, channel, grad, count, dtype, param, master, s1, s2, h, 1.f, nullptr, nullptr, false);
   API_END(-1)
 }
 

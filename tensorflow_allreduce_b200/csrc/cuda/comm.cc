@@ -505,9 +505,8 @@ void Comm::allgatherv(int channel, const void* in, size_t bytes, void* out_symm,
 }
 
 Algo Comm::fused_step(int channel, void* grad, size_t count, DType dtype, void* param, float* master, float* s1, float* s2,
-                      const OptHyper& h, float scale, cudaStream_t stream_override, bool beside_compute) {
+                      const OptHyper& h, float scale, cudaStream_t s, bool beside_compute) {
   CUDA_RT(cudaSetDevice(device_));
-  cudaStream_t s = stream_override ? stream_override : streams_[channel];
   const size_t bytes = count * dtype_size(dtype);
   if (count == 0) return Algo::TWO_SHOT;
   ArArgs a;

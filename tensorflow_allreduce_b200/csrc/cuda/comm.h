@@ -106,7 +106,7 @@ class Comm {
   // `beside_compute`: the launch shares the GPU with the backward pass; its grid is capped so
   // that all of its blocks can be resident together (see choose_blocks).
   Algo fused_step(int channel, void* grad, size_t count, DType dtype, void* param, float* master, float* s1, float* s2,
-                  const OptHyper& h, float scale, cudaStream_t stream_override, bool beside_compute = false);
+                  const OptHyper& h, float scale, cudaStream_t s, bool beside_compute = false);
 
   // Device array of kProfStamps time stamps that the next reduction launches fill in (null: off).
   void set_profile(unsigned long long* stamps) { prof_ = stamps; }

@@ -418,6 +418,9 @@ class DistributedOptimizer(torch.optim.Optimizer):
     def _alias_state(self):
         """Flat optimizer state per arena, exposed per parameter in `optimizer.state` under the
         keys torch uses, so `state_dict()` / `load_state_dict()` keep working."""
+        if self._kind == 2 and not hasattr(self, "_steps"):
+            self._steps = [torch.zeros(len(g["params"]), dtype=torch.float32) for g in self.param_groups]
+            self._step_index = {p: i for g in self.param_groups for i, p in enumerate(g["params"])}
         for ar in self._arenas:
             g = self.param_groups[ar.group_index]
             dev = ar.grad.device
@@ -449,8 +452,12 @@ class DistributedOptimizer(torch.optim.Optimizer):
                         if old is not None and old.data_ptr() != flat[sl].data_ptr():
                             flat[sl].copy_(old.reshape(-1).float())
                         st[key] = flat[sl].view(p.shape)
-                    if "step" not in st:
-                        st["step"] = torch.tensor(0.0, dtype=torch.float32)
+                    # the step counters of a group's parameters are elements of one tensor: one write per step
+                    steps, i = self._steps[b.group_index], self._step_index[p]
+                    old = st.get("step")
+                    if old is not None and not (torch.is_tensor(old) and old.data_ptr() == steps[i].data_ptr()):
+                        steps[i] = float(old)
+                    st["step"] = steps[i]
         for gi, g in enumerate(self.param_groups):
             steps = [float(self.state[p]["step"]) for p in g["params"] if p in self.state and "step" in self.state[p]]
             if steps:
@@ -588,8 +595,13 @@ class DistributedOptimizer(torch.optim.Optimizer):
     def _finish_reduction(self):
         """Launch the buckets that have not gone yet and make the current stream wait for all."""
         # Buckets whose parameters received no gradient in this pass are reduced now (zeros).
-        for b in self._buckets[self._next_bucket:]:
-            self._launch(b)
+        rest = self._buckets[self._next_bucket:]
+        sampled = self._timing_every and self._iteration % self._timing_every == 0     # then every bucket is timed by itself
+        if rest and self._kind and self._world == 1 and not sampled:
+            self._launch_rest_alone(rest)
+        else:
+            for b in rest:
+                self._launch(b)
         self._next_bucket = len(self._buckets)
         cur = torch.cuda.current_stream()
         for b in self._buckets:
@@ -600,6 +612,28 @@ class DistributedOptimizer(torch.optim.Optimizer):
         for b in self._buckets:
             if b.launched:
                 cur.wait_event(b.done_event)
+
+    def _launch_rest_alone(self, rest):
+        """The updates that are left in a group of one rank: no peer has to see the same sequence of launches and no backward
+        pass is left to overlap, so neighbouring ranges of an arena go out as one launch, on the current stream. (25 launches
+        of 28 MB on the private stream left gaps of 3 us each and two event round trips.)"""
+        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        order = sorted(rest, key=lambda b: (self._arenas.index(b.arena), b.lo))
+        i = 0
+        while i < len(order):
+            ar, lo, hi = order[i].arena, order[i].lo, order[i].hi
+            gap = _ALIGN_BYTES // ar.grad.element_size()     # alignment padding between two units, all zeros
+            first = order[i]
+            i += 1
+            while i < len(order) and order[i].arena is ar and order[i].lo - hi < gap:
+                hi = order[i].hi
+                i += 1
+            ptr = [C.c_void_p(t.data_ptr() + lo * t.element_size()) if t is not None else None
+                   for t in (ar.grad, ar.param, ar.master, ar.state1, ar.state2)]
+            core._call(_lib.lib().bc_fused_step_alone(_FUSED_CHANNEL, stream, ptr[0], hi - lo, core._DTYPES[ar.dtype], *ptr[1:],
+                                                      C.byref(self._hyper(first))), "update")
+            self._launched_any = True
+            self.launch_count += 1
 
     @torch.no_grad()
     def synchronize(self):
@@ -639,10 +673,7 @@ class DistributedOptimizer(torch.optim.Optimizer):
                 self._step_count[gi] += 1
                 self._momentum_live[gi] = True
                 if self._kind == 2:
-                    for p in g["params"]:
-                        st = self.state.get(p)
-                        if st is not None and "step" in st:
-                            st["step"] = torch.tensor(float(self._step_count[gi]), dtype=torch.float32)
+                    self._steps[gi].fill_(float(self._step_count[gi]))
         else:
             self._optimizer.step()
         for b in self._buckets:
