@@ -47,6 +47,8 @@
 // (bounded) for its own MMAs in flight, frees its tensor memory and returns.
 #include "gru_persistent.h"
 
+#include "tcgen05_prims.cuh"
+
 #include <algorithm>
 #include <atomic>
 
@@ -55,13 +57,15 @@ namespace gpu {
 
 namespace {
 
+using namespace tc;
+
 constexpr int kUnits = 16;            // hidden units per block
 constexpr int kKTile = 32;            // fp32 elements in one 128-byte swizzle row
 constexpr int kGateThreads = 256;     // eight warps: accumulator read-back, exchange, gate math
 constexpr int kLoadThreads = 256;     // eight warps: poll the operand words and put them into shared memory
 constexpr int kThreads = kGateThreads + kLoadThreads + 32;   // and the warp that issues the MMAs
 constexpr int kMaxBlocksPerDir = 64;  // H / 16 at H = 1024
-constexpr int kTmemCols = 512;
+constexpr uint32_t kTmemCols = 512;
 constexpr int kLoadBytes = kLoadThreads * 32;   // operand bytes that one load of every loader thread brings
 constexpr int kLoadsPerGroup = 2;     // loads of a thread per pipeline group (one mbarrier each)
 constexpr int kMaxGroups = 8;         // of a step: 32 K tiles of 32 batch rows, H = 1024 unsplit
@@ -85,72 +89,12 @@ struct Params {
   unsigned long long* prof;   // optional: 8 time stamps per step of block (0, 0), for tuning
 };
 
-// ---- PTX wrappers ---------------------------------------------------------------------------
+// ---- PTX wrappers beside those of tcgen05_prims.cuh ---------------------------------------------
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned long long gtimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 __device__ __forceinline__ uint32_t clock32() {
   uint32_t c;
   asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
   return c;
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return ok != 0;
-}
-// Bounded wait for the phase with the given parity; also gives up when `abort_flag` is raised.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned long long timeout_ns, const volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = gtimer();
-  uint32_t spins = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if (((++spins) & 63) == 0) {
-      if (abort_flag && *abort_flag) return false;
-      if (gtimer() - t0 > timeout_ns) return false;
-    }
-  }
-  return true;
-}
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D[m, n] (+)= A[m, k] * B[n, k], A in tensor memory / in shared memory.
-__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_mma_ss(uint32_t d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // N consecutive columns of this thread's tensor-memory lane: the packs that one warp reads back (see `send` below).
 template <int N> __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t* r);
@@ -170,14 +114,6 @@ template <> __device__ __forceinline__ void tc_ld<9>(uint32_t taddr, uint32_t* r
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8])
       : "r"(taddr), "r"(taddr + 8) : "memory");
 }
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const float* v) {
-  const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-
 // Words that travel between blocks.
 __device__ __forceinline__ void st_word(uint32_t* p, uint32_t v) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 // 32 bytes per request: a strong load costs L2 the same whatever its width (fresh lines, 32 KB per block and 128 blocks:
@@ -217,35 +153,7 @@ __device__ __forceinline__ bool stale(const Words& v, uint32_t tag) {
   return (d & kTagMask) != 0;
 }
 
-// Shared-memory matrix descriptor of a K-major operand tile stored as rows of 128 bytes with the
-// 128-byte swizzle (16-byte chunk c of row r sits at chunk c ^ (r & 7)): groups of 8 rows are 1024
-// bytes apart; the leading-dimension offset is unused because a tile is one swizzle atom wide.
-__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);   // start address
-  d |= (uint64_t)(1024u >> 4) << 32;              // stride between 8-row groups
-  d |= (uint64_t)1 << 46;                         // descriptor version of sm_100
-  d |= (uint64_t)2 << 61;                         // 128-byte swizzle
-  return d;
-}
-
-// The gate functions are on the critical path of every step and issue-bound (eight warps run 512 of each), so they are
-// made of the fewest instructions that keep fp32 accuracy: a reciprocal with one Newton step instead of a division.
-__device__ __forceinline__ float recip(float y) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
-  return fmaf(r, fmaf(-y, r, 1.f), r);
-}
-__device__ __forceinline__ float sigmoidf_(float x) { return recip(1.f + __expf(fminf(-x, 80.f))); }
-// 1 - 2 / (1 + e^2x); near zero, where that cancels, the Taylor series up to x^9 (its error at 0.3 is 1e-8).
-__device__ __forceinline__ float tanhf_(float x) {
-  const float t = 1.f - 2.f * recip(1.f + __expf(fminf(2.f * x, 80.f)));
-  const float q = x * x;
-  float c = fmaf(q, 62.f / 2835.f, -17.f / 315.f);
-  c = fmaf(q, c, 2.f / 15.f);
-  c = fmaf(q, c, -1.f / 3.f);
-  return fabsf(x) < 0.3f ? fmaf(x * q, c, x) : t;
-}
+__device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf(-x)); }
 
 // Barrier 1: all gate and loader warps have read the accumulator and sent their part of it; the loaders only arrive.
 __device__ __forceinline__ void sent_sync() { asm volatile("barrier.cta.sync 1, 512;" ::: "memory"); }
@@ -271,7 +179,7 @@ __host__ __device__ inline Plan make_plan(int C, int nb, int H) {
   p.kq = (BWD ? 3 * H : H) / C;
   p.ntile = (p.kq + kKTile - 1) / kKTile;
   p.m = rows > 64 ? 128 : 64;
-  const int room = kTmemCols - nb;                 // the accumulator takes the first nb columns
+  const int room = (int)kTmemCols - nb;                 // the accumulator takes the first nb columns
   p.k_tmem = p.kq <= room ? p.kq : room / kKTile * kKTile;
   p.x_bytes = p.ntile * nb * 128;
   p.w_bytes = (p.kq - p.k_tmem + kKTile - 1) / kKTile * p.m * 128;
@@ -341,8 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kThreads / 32 - 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)kTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    tmem_alloc(tmem_slot, kTmemCols);
   }
 
   // The part of the ring that this block writes (both slots) and the partial sums that it will
@@ -400,9 +307,9 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       for (int i = 0; i < 16; i++) v[i] = 0.f;
       if (row_ok) load_weights16<BWD>(w, H, C, grp, q, pl.kq, lane_row, k0, v);
       __syncwarp();
-      tc_st16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(NB + k0), v);
+      tmem_st16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(NB + k0), v);
     }
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tmem_st_wait();
     for (int i = tid; i < pl.m * ((pl.kq - pl.k_tmem) / 16); i += 256) {
       const int r = i % pl.m, k = (i / pl.m) * 16;                     // counted from k_tmem
       float v[16];
@@ -712,7 +619,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
           const float hn = bias_n + acc[2][j];
           const float r_ = sigmoidf_(gx[0][j] + (bias_r + acc[0][j]));
           const float z = sigmoidf_(gx[1][j] + (bias_z + acc[1][j]));
-          const float n = tanhf_(gx[2][j] + r_ * hn);
+          const float n = tanhf(gx[2][j] + r_ * hn);
           carry[j] = n + z * (carry[j] - n);
           keep[j] = make_float4(r_, z, n, hn);
         }
@@ -829,7 +736,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   if (warp == kThreads / 32 - 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTmemCols) : "memory");
+    tmem_free(tmem, kTmemCols);
 }
 
 // ---- host side ------------------------------------------------------------------------------
