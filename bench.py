@@ -70,7 +70,7 @@ def build_model(name: str, device, batch: int, persistent_rnn: bool = True, fuse
     if name == "ds2":
         from tensorflow_allreduce_b200.models import ds2
 
-        cfg = ds2.DS2Config(persistent_rnn=persistent_rnn, fused_norm=fused_norm)
+        cfg = ds2.DS2Config(persistent_rnn=persistent_rnn, fused_norm=fused_norm, row_conv=fused_norm)
         model = ds2.DeepSpeech2(cfg).to(device)
         model.rnn.flatten_parameters()
         b = batch or 32

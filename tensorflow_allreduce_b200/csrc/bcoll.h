@@ -170,6 +170,17 @@ int bc_gru_forward(int T, int B, int H, int ndir, const float* w_hh0, const floa
 int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* y, const float* rsv,
                     const float* dy, float* dg, float* db, void* scratch, unsigned* status, double timeout_s, void* stream);
 
+/* Row convolutions (csrc/cuda/conv_rows.h): 32 output channels, stride (2, 1) with 32 input channels or (2, 2) with one.
+ * `dims` = {N, Cin, H, W, KH, KW, ph, pw, stride_w}; `scratch` = bc_conv_scratch_bytes() bytes, contents irrelevant;
+ * `status` as above. */
+int bc_conv_supported(int device, const int* dims);
+long long bc_conv_scratch_bytes(const int* dims);
+int bc_conv_forward(const int* dims, const float* x, const float* w, float* y, void* scratch, unsigned* status, double timeout_s, void* stream);
+int bc_conv_backward_input(const int* dims, const float* dy, const float* w, float* dx, void* scratch, unsigned* status, double timeout_s,
+                           void* stream);
+int bc_conv_backward_weight(const int* dims, const float* x, const float* dy, float* dw, void* scratch, unsigned* status, double timeout_s,
+                            void* stream);
+
 /* Training-mode batch normalisation of [N, C, HW] fp32 activations fused with the clipped ReLU behind it
  * (y = clamp(bn(x), 0, clip_hi)); csrc/cuda/bn_clip.h. `acc` = scratch of 2 * (C + 1024) doubles; running_* and `batches` (a counter that goes up by one) may be NULL.
  * These need no initialised group. */

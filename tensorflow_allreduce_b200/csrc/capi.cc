@@ -14,6 +14,7 @@
 
 #include "cuda/comm.h"
 #include "cuda/bn_clip.h"
+#include "cuda/conv_rows.h"
 #include "cuda/gru_persistent.h"
 #include "runtime/runtime.h"
 #include "runtime/two_level.h"
@@ -586,6 +587,39 @@ int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const flo
   const float* w[2] = {w_hh0, w_hh1};
   check_cuda(gpu::gru_persistent_backward(d, w, y, rsv, dy, dg, db, scratch, status, timeout_s, (cudaStream_t)stream),
              "persistent GRU backward launch");
+  return 0;
+  API_END(-1)
+}
+
+// ---- row convolutions --------------------------------------------------------------------------------
+
+static gpu::ConvDims conv_dims(const int* v) { return gpu::ConvDims{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]}; }
+
+int bc_conv_supported(int device, const int* dims) { return gpu::conv_rows_supported(conv_dims(dims), device) ? 1 : 0; }
+
+long long bc_conv_scratch_bytes(const int* dims) { return (long long)gpu::conv_rows_scratch_bytes(conv_dims(dims)); }
+
+int bc_conv_forward(const int* dims, const float* x, const float* w, float* y, void* scratch, unsigned* status, double timeout_s, void* stream) {
+  API_BEGIN
+  check_cuda(gpu::conv_rows_forward(conv_dims(dims), x, w, y, scratch, status, timeout_s, (cudaStream_t)stream), "row convolution launch");
+  return 0;
+  API_END(-1)
+}
+
+int bc_conv_backward_input(const int* dims, const float* dy, const float* w, float* dx, void* scratch, unsigned* status, double timeout_s,
+                           void* stream) {
+  API_BEGIN
+  check_cuda(gpu::conv_rows_backward_input(conv_dims(dims), dy, w, dx, scratch, status, timeout_s, (cudaStream_t)stream),
+             "row convolution input gradient launch");
+  return 0;
+  API_END(-1)
+}
+
+int bc_conv_backward_weight(const int* dims, const float* x, const float* dy, float* dw, void* scratch, unsigned* status, double timeout_s,
+                            void* stream) {
+  API_BEGIN
+  check_cuda(gpu::conv_rows_backward_weight(conv_dims(dims), x, dy, dw, scratch, status, timeout_s, (cudaStream_t)stream),
+             "row convolution weight gradient launch");
   return 0;
   API_END(-1)
 }

@@ -204,6 +204,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
         const int t = u / R, r = u % R;
         uint32_t v[32];
         tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(u * 32), v);
+        if (lo > hi) {             // no input row meets these output rows (trailing rows of an input gradient)
+#pragma unroll
+          for (int c = 0; c < 32; c++) v[c] = 0u;
+        }
         const int col = w0 + t * 128 + quarter * 32 + lane;
         if (o0 + r < p.Ho && col < p.Wo) {
           float* o = p.y + (size_t)n * kCo * oplane + (size_t)(o0 + r) * p.Wo + col;
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
 // HB = 8: one input channel, 16 shifts, M row = (input row) * 16 + shift. Kernel row kh = 2 m + parity; an input row block at
 // h, with e = (h + ph - parity) / 2, meets output row oh = e - m' where m' = m - (row of the block).
 template <int HB> struct WgradShape {
-  static constexpr int kCi = HB == 1 ? 32 : 1, kShifts = HB == 1 ? 4 : 16, kStride = HB == 1 ? 1 : 2;
+  static constexpr int kCi = HB == 1 ? 32 : 1;
   static constexpr int kAStages = HB == 1 ? 4 : 2, kRing = HB == 1 ? 16 : 32;
   static constexpr int smem = 1024 + kAStages * 128 * kRow + kRing * kCo * kRow + 256;
 };
@@ -591,7 +595,7 @@ cudaError_t run_wgrad(const ConvDims& d, const float* x, const float* dy, float*
 bool dims_ok(const ConvDims& d) {
   if (d.N < 1 || d.N > 65535 || d.H < 1 || d.W < 1 || d.KH < 1 || d.KW < 1 || d.KW > 16 || d.ph < 0 || d.pw < 0 || d.ph >= d.KH || d.pw >= d.KW) return false;
   if (d.H + 2 * d.ph < d.KH || d.W + 2 * d.pw < d.KW || d.H > 4096 || d.W > (1 << 20)) return false;
-  if (d.Cin == 32) return d.stride_w == 1 && d.KH <= 2 * kMaxM - 4;                  // the ring of the weight gradient holds its window
+  if (d.Cin == 32) return d.stride_w == 1 && (d.KH + 1) / 2 <= 13;                   // the ring of the weight gradient holds its window
   return d.Cin == 1 && d.stride_w == 2 && d.ph % 2 == 0 && (d.KH + 1) / 2 + 7 <= 2 * kMaxM;
 }
 

@@ -237,6 +237,74 @@ std::vector<int> gru_devices() {
   return out;
 }
 
+// ---- row convolutions ---------------------------------------------------------------------------
+
+std::atomic<long long> g_conv_launches{0};
+
+struct Conv {
+  int v[9];
+  Conv(const Tensor& x, const Tensor& w, int64_t ph, int64_t pw)
+      : v{(int)x.size(0), (int)x.size(1), (int)x.size(2), (int)x.size(3), (int)w.size(2), (int)w.size(3), (int)ph, (int)pw, x.size(1) == 1 ? 2 : 1} {}
+  int64_t Ho() const { return (v[2] + 2 * v[6] - v[4]) / 2 + 1; }
+  int64_t Wo() const { return (v[3] + 2 * v[7] - v[5]) / v[8] + 1; }
+  Tensor scratch(const Tensor& like) const { return at::empty({(int64_t)bc_conv_scratch_bytes(v)}, like.options().dtype(at::kByte)); }
+};
+
+struct ConvRows : torch::autograd::Function<ConvRows> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, int64_t ph, int64_t pw) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Conv c(x, w, ph, pw);
+    const Tensor wc = w.contiguous(), scratch = c.scratch(x);
+    Tensor y = at::empty({x.size(0), 32, c.Ho(), c.Wo()}, x.options());
+    check(bc_conv_forward(c.v, ptr(x), ptr(wc), ptr(y), scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, stream_of(x)), "bc_conv_forward");
+    g_conv_launches++;
+    ctx->save_for_backward({x, wc});
+    ctx->saved_data["ph"] = ph;
+    ctx->saved_data["pw"] = pw;
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1];
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t ph = ctx->saved_data["ph"].toInt(), pw = ctx->saved_data["pw"].toInt();
+    const Conv c(x, w, ph, pw);
+    const Tensor dy = grads[0].contiguous(), scratch = c.scratch(x);
+    unsigned* status = (unsigned*)gru_status(x);
+    Tensor dx, dw;
+    if (ctx->needs_input_grad(1)) {
+      dw = at::empty_like(w);
+      check(bc_conv_backward_weight(c.v, ptr(x), ptr(dy), ptr(dw), scratch.data_ptr(), status, g_gru_timeout_s, stream_of(x)), "bc_conv_backward_weight");
+      g_conv_launches++;
+    }
+    if (ctx->needs_input_grad(0)) {
+      if (x.size(1) == 32) {
+        dx = at::empty_like(x);
+        check(bc_conv_backward_input(c.v, ptr(dy), ptr(w), ptr(dx), scratch.data_ptr(), status, g_gru_timeout_s, stream_of(x)), "bc_conv_backward_input");
+        g_conv_launches++;
+      } else {       // the spectrogram's gradient is not part of training
+        const int64_t sw = c.v[8];
+        dx = std::get<0>(at::convolution_backward(dy, x, w, c10::nullopt, {2, sw}, {ph, pw}, {1, 1}, false, {0, 0}, 1, {true, false, false}));
+      }
+    }
+    return {dx, dw, Tensor(), Tensor()};
+  }
+};
+
+bool conv_supported(const Tensor& x, const Tensor& w, int64_t ph, int64_t pw) {
+  if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != at::kFloat || w.scalar_type() != at::kFloat || x.dim() != 4 || w.dim() != 4 ||
+      !x.is_contiguous() || w.size(0) != 32 || w.size(1) != x.size(1) || x.size(0) > 65535)
+    return false;
+  const Conv c(x, w, ph, pw);
+  return bc_conv_supported(x.device().index(), c.v) == 1;
+}
+
+Tensor conv_rows(const Tensor& x, const Tensor& w, int64_t ph, int64_t pw) {
+  TORCH_CHECK(conv_supported(x, w, ph, pw), "conv_rows does not cover this convolution");
+  return ConvRows::apply(x, w, ph, pw);
+}
+
 // ---- collectives of a group of one --------------------------------------------------------------
 
 int dtype_code(at::ScalarType t) {
@@ -276,5 +344,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gru_set_timeout", [](double s) { g_gru_timeout_s = s; });
   m.def("gru_take_status", &gru_take_status);
   m.def("gru_devices", &gru_devices);
+  m.def("conv_supported", &conv_supported);
+  m.def("conv_rows", &conv_rows);
+  m.def("conv_launches", [] { return g_conv_launches.load(); });
   m.def("allreduce_alone", &allreduce_alone);
 }

@@ -4,8 +4,9 @@ Two 2-D convolutions over (frequency, time) with batch norm and clipped ReLU, a 
 bidirectional GRU layers, a linear layer to the character classes and CTC loss. The reference
 ships no such model; its pieces there are Conv2D/cuDNN, FusedBatchNorm, Relu6-style clipping,
 GRU cells (tensorflow/contrib/rnn/kernels/gru_ops.h:69-119) or CudnnRNN, and a CPU-only CTC loss
-(tensorflow/core/kernels/ctc_loss_op.cc:167). Here the convolutions, the output layer and the loss
-are plain torch.nn modules on cuDNN/cuBLAS; batch norm and the clipped ReLU behind it are one
+(tensorflow/core/kernels/ctc_loss_op.cc:167). Here the output layer and the loss are plain torch.nn
+modules on cuBLAS; the convolutions run on the library's tcgen05 kernels where these cover them
+(`ops/conv_rows.py`, else cuDNN); batch norm and the clipped ReLU behind it are one
 module on the library's two-pass kernels (`ops/bn_clip.py`); the GRU stack keeps its `nn.GRU` module
 and parameters but, on a GPU that supports them, is evaluated by the library's persistent
 tcgen05 kernels (`ops/persistent_gru.py`); the gradient reduction and update around the model are
@@ -31,6 +32,7 @@ class DS2Config:
     label_len: int = 100
     persistent_rnn: bool = True  # run the GRU stack on the library's persistent tcgen05 kernels when they support the shape
     fused_norm: bool = True      # batch norm + clipped ReLU as one module on the library's two-pass kernels (ops/bn_clip.py)
+    row_conv: bool = True        # convolutions on the library's tcgen05 kernels where they cover them (ops/conv_rows.py)
 
 
 class DeepSpeech2(nn.Module):
@@ -47,10 +49,14 @@ class DeepSpeech2(nn.Module):
                 return [BatchNormClip2d(c, clip=20.0), nn.Identity()]
             return [nn.BatchNorm2d(c), nn.Hardtanh(0.0, 20.0, inplace=True)]
 
+        if cfg.row_conv:
+            from ..ops.conv_rows import RowConv2d as Conv2d
+        else:
+            Conv2d = nn.Conv2d
         self.conv = nn.Sequential(
-            nn.Conv2d(1, c, kernel_size=(41, 11), stride=(2, 2), padding=(20, 5), bias=False),
+            Conv2d(1, c, kernel_size=(41, 11), stride=(2, 2), padding=(20, 5), bias=False),
             *norm_act(),
-            nn.Conv2d(c, c, kernel_size=(21, 11), stride=(2, 1), padding=(10, 5), bias=False),
+            Conv2d(c, c, kernel_size=(21, 11), stride=(2, 1), padding=(10, 5), bias=False),
             *norm_act(),
         )
         f = (cfg.n_freq + 2 * 20 - 41) // 2 + 1

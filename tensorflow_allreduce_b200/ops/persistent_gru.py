@@ -46,6 +46,8 @@ def check_status(device=None) -> None:
             continue
         code = e.gru_take_status(idx)
         if code:
+            if code & 8:
+                raise RuntimeError(f"a row convolution timed out on cuda:{idx} (status 0x{code:x}); its outputs are incomplete")
             raise RuntimeError(f"a persistent GRU kernel timed out on cuda:{idx} (status 0x{code:x}); its outputs are incomplete")
 
 
