@@ -153,7 +153,30 @@ __device__ __forceinline__ bool stale(const Words& v, uint32_t tag) {
   return (d & kTagMask) != 0;
 }
 
-__device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf(-x)); }
+// The gate functions are on the critical path of every step and bound by instruction issue: with `tanhf` and IEEE divisions a
+// step took 0.6 us longer (H = 1024, B = 32). Their errors stay within a few units in the last place, far
+// below the TF32 rounding of the product in front of them.
+__device__ __forceinline__ float exp_(float x) {      // 2^(x log2 e)
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.44269504f));
+  return y;
+}
+__device__ __forceinline__ float div_(float a, float b) {
+  float y;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ float sigmoidf_(float x) { return div_(1.f, 1.f + exp_(-x)); }
+// 1 - 2 / (1 + e^2x); where that cancels, Lambert's continued fraction of tanh cut behind its fifth partial denominator,
+// x (945 + 105 q + q^2) / (945 + 420 q + 15 q^2) with q = x^2, whose error at 0.625 is below 1e-9.
+__device__ __forceinline__ float tanhf_(float x) {
+  const float q = x * x;
+  const bool small = q < 0.39f;
+  const float num = small ? x * fmaf(q, q + 105.f, 945.f) : -2.f;
+  const float den = small ? fmaf(q, fmaf(q, 15.f, 420.f), 945.f) : 1.f + exp_(2.f * x);
+  const float v = div_(num, den);
+  return small ? v : 1.f + v;
+}
 
 // Barrier 1: all gate and loader warps have read the accumulator and sent their part of it; the loaders only arrive.
 __device__ __forceinline__ void sent_sync() { asm volatile("barrier.cta.sync 1, 512;" ::: "memory"); }
@@ -619,7 +642,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
           const float hn = bias_n + acc[2][j];
           const float r_ = sigmoidf_(gx[0][j] + (bias_r + acc[0][j]));
           const float z = sigmoidf_(gx[1][j] + (bias_z + acc[1][j]));
-          const float n = tanhf(gx[2][j] + r_ * hn);
+          const float n = tanhf_(gx[2][j] + r_ * hn);
           carry[j] = n + z * (carry[j] - n);
           keep[j] = make_float4(r_, z, n, hn);
         }
