@@ -67,8 +67,7 @@ constexpr int kThreads = kGateThreads + kLoadThreads + 32;   // and the warp tha
 constexpr int kMaxBlocksPerDir = 64;  // H / 16 at H = 1024
 constexpr uint32_t kTmemCols = 512;
 constexpr int kLoadBytes = kLoadThreads * 32;   // operand bytes that one load of every loader thread brings
-constexpr int kLoadsPerGroup = 2;     // loads of a thread per pipeline group (one mbarrier each)
-constexpr int kMaxGroups = 8;         // of a step: 32 K tiles of 32 batch rows, H = 1024 unsplit
+constexpr int kMaxGroups = 8;         // pipeline groups (one mbarrier each) of a step: 32 K tiles of 32 batch rows in pairs of loads
 constexpr int kMinSmem = 120 * 1024;  // more than half of an SM's shared memory: one block per SM, since a block takes all of tensor memory
 
 struct Params {
@@ -229,13 +228,15 @@ __device__ __forceinline__ void load_weights16(const float* w, int H, int C, int
   }
 }
 
-// BWD: pass; C: blocks per group; NB: N of the MMA (16 or 32, at least the batch).
+// BWD: pass; C: blocks per group; NB: N of the MMA (16 or 32, at least the batch); kLoadsPerGroup: loads of a loader thread per
+// pipeline group. With five loads or more, groups of four, one in flight, win (H = 1024, B = 32: forward 3.81 -> 3.72, backward 4.39 ->
+// 4.24 us per step: fewer polls of words that are not there yet); with fewer, pairs do (forward H = 512: 2.87 against 2.97).
 //
 // Three kinds of warps, so that no work off the chain of a step (output stores, prefetches) delays the next
 // product: gate warps, loader warps, and one warp that issues the MMAs. One barrier each says that
 // the operand is in shared memory (full[group]: loaders -> MMA), that the accumulator is complete (done:
 // MMA -> all), that it has been read (read: all -> MMA), and that this block has published (published: gates -> loaders).
-template <bool BWD, int C, int NB>
+template <bool BWD, int C, int NB, int kLoadsPerGroup>
 __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     const int tiles_mine = chunk < last_chunks ? pl.ntile : pl.ntile - 1;
     const int mine = b < B && kt0 < tiles_mine ? (tiles_mine - kt0 + kTilesPerLoad - 1) / kTilesPerLoad : 0;
     const uint32_t pause = (uint32_t)(pl.ntile * B * 128) / 80;      // cycles
-    constexpr int kSpan = 3;           // groups whose loads are in flight together
+    constexpr int kSpan = kLoadsPerGroup == 4 ? 1 : 3;           // groups whose loads are in flight together
     bool good = true;
     // Every step is gone through to the end even when a wait has run out (the waits then end at once): the gate warps count
     // on the arrivals.
@@ -803,14 +804,14 @@ constexpr size_t kSyncBytes = 1024;
 // a member may be half empty.
 size_t ring_bytes(const GruDims& d) { return (size_t)d.ndir * 2 * (3 * d.H + 16 * 16) * 32 * 4; }
 
-template <bool BWD, int C, int NB>
-cudaError_t launch_as(const Params& p, cudaStream_t stream) {
+template <bool BWD, int C, int NB, int LPG>
+cudaError_t launch_with(const Params& p, cudaStream_t stream) {
   const GruDims& d = p.d;
   const Plan pl = make_plan<BWD>(C, NB, d.H);
-  auto kernel = gru_persistent_kernel<BWD, C, NB>;
+  auto kernel = gru_persistent_kernel<BWD, C, NB, LPG>;
   const int smem = std::max(pl.smem(), kMinSmem);
   dim3 grid(d.H / kUnits, d.ndir), block(kThreads);
-  if (grid.x > (unsigned)kMaxBlocksPerDir || grid.x % C != 0 || (pl.ntile + 64 / NB - 1) / (64 / NB) > kLoadsPerGroup * kMaxGroups) return cudaErrorInvalidValue;
+  if (grid.x > (unsigned)kMaxBlocksPerDir || grid.x % C != 0 || (pl.ntile + 64 / NB - 1) / (64 / NB) > LPG * kMaxGroups) return cudaErrorInvalidValue;
   // The attribute belongs to a device: set once for each, to all that a block can have.
   static std::atomic<uint64_t> granted{0};
   int dev = 0;
@@ -822,6 +823,12 @@ cudaError_t launch_as(const Params& p, cudaStream_t stream) {
   }
   void* args[] = {(void*)&p};
   return cudaLaunchCooperativeKernel((const void*)kernel, grid, block, args, (size_t)smem, stream);
+}
+
+template <bool BWD, int C, int NB>
+cudaError_t launch_as(const Params& p, cudaStream_t stream) {
+  const int loads = (make_plan<BWD>(C, NB, p.d.H).ntile + 64 / NB - 1) / (64 / NB);
+  return loads >= 5 ? launch_with<BWD, C, NB, 4>(p, stream) : launch_with<BWD, C, NB, 2>(p, stream);
 }
 
 template <bool BWD>
