@@ -523,18 +523,37 @@ __global__ void __launch_bounds__(256) wgrad_sum_kernel(const float* __restrict_
 // ---- host side -------------------------------------------------------------------------------------
 
 int tiles_of(int cols) { return std::min((cols + 127) / 128, kMaxCols / 128); }
-// Output rows per block: as many as tensor memory holds (16 units of 32 columns over all tiles), at most N = 256 per MMA.
-int rows_of(int T) { return std::min(16 / T, 8); }
-
-size_t table_bytes(int mode, const ConvDims& d, int R) {
-  const int tables = mode == GATHER ? 1 : d.KW * (mode == FORWARD ? 2 : 1);
-  return (size_t)tables * table_rows(mode, d.KH, R) * kCo * kRow;
-}
-
 int sm_count() {
   int dev = 0, n = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
   return n;
+}
+
+// Output rows per block, at most what tensor memory holds (16 units of 32 columns over all tiles) and N = 256 per MMA. More
+// rows share an input row's loads and make wider MMAs, but also compute more rows than the kernel is high and leave fewer
+// blocks: the number that needs the fewest cycles in the fullest SM. An MMA measured 110 cycles up to 5 rows, 17 per row above; conv 1
+// is bound by its loads, 1340 cycles per row and tile. (32 -> 32 channels, 81 x 50, 4 images: 5 blocks of 8 rows 156 us, chosen rows
+// 93 us; 32 images of 81 x 350 stay at 5 rows: 470 us, with 4 rows for the input gradient 466 instead of 393 us.)
+int rows_of(int mode, const ConvDims& d, int Ho, int Wo, int sms) {
+  const int T = tiles_of(Wo);
+  int best = 1;
+  double least = 0;
+  for (int R = 1; R <= std::min(16 / T, 8); R++) {
+    const int rows = mode == FORWARD ? d.KH + 2 * (R - 1) : mode == DGRAD ? (d.KH + R) / 2 : half_taps(d.KH) + R - 1;
+    const long blocks = (long)d.N * ((Ho + R - 1) / R) * ((Wo + kMaxCols - 1) / kMaxCols);
+    const double row = mode == GATHER ? std::max(1340, 4 * 17 * R) : d.KW * 4 * std::max(110, 17 * R);
+    const double cycles = (double)((blocks + sms - 1) / sms) * (5000 + rows * row * T);
+    if (R == 1 || cycles < least) {
+      least = cycles;
+      best = R;
+    }
+  }
+  return best;
+}
+
+size_t table_bytes(int mode, const ConvDims& d, int R) {
+  const int tables = mode == GATHER ? 1 : d.KW * (mode == FORWARD ? 2 : 1);
+  return (size_t)tables * table_rows(mode, d.KH, R) * kCo * kRow;
 }
 
 template <int HB> int wgrad_kinds(const ConvDims& d) { return 2 * (HB == 1 ? (d.KW + 3) / 4 : 2); }
@@ -553,7 +572,7 @@ cudaError_t run_rows(const ConvDims& d, const float* x, const float* w, float* y
                      uint32_t* status, double timeout_s, cudaStream_t stream) {
   RowsParams p;
   p.T = tiles_of(Wo);
-  p.R = rows_of(p.T);
+  p.R = rows_of(MODE, d, Ho, Wo, sm_count());
   p.x = x;
   p.y = y;
   p.w = (const char*)scratch;
