@@ -828,7 +828,9 @@ cudaError_t launch_with(const Params& p, cudaStream_t stream) {
 template <bool BWD, int C, int NB>
 cudaError_t launch_as(const Params& p, cudaStream_t stream) {
   const int loads = (make_plan<BWD>(C, NB, p.d.H).ntile + 64 / NB - 1) / (64 / NB);
-  return loads >= 5 ? launch_with<BWD, C, NB, 4>(p, stream) : launch_with<BWD, C, NB, 2>(p, stream);
+  if constexpr (BWD || C > 1)            // alone in its group a forward block never has more than four
+    if (loads >= 5) return launch_with<BWD, C, NB, 4>(p, stream);
+  return launch_with<BWD, C, NB, 2>(p, stream);
 }
 
 template <bool BWD>

@@ -40,16 +40,24 @@ class BatchNormClip2d(torch.nn.BatchNorm2d):
 
     def _fused_ok(self, x: torch.Tensor) -> bool:
         return (self.training and x.is_cuda and x.dtype == torch.float32 and x.dim() == 4 and x.is_contiguous() and self.affine
-                and self.weight.dtype == torch.float32 and self.momentum is not None
-                and (not self.track_running_stats or self.running_mean is not None) and x.numel() > 0
-                and x.numel() // (x.shape[0] * x.shape[1]) < 2 ** 31)
+                and self.momentum is not None and (not self.track_running_stats or self._buffers.get("running_mean") is not None)
+                and x.numel() > 0 and x.shape[2] * x.shape[3] < 2 ** 31)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if not self._fused_ok(x):
+        # Parameters and buffers are taken from the module's dictionaries where they are there: an attribute of a module
+        # costs most of a microsecond, and a small batch is bound by the host. (A parametrised weight is not there.)
+        weight = self._parameters.get("weight")
+        if weight is None and self.affine:
+            weight = self.weight
+        if not self._fused_ok(x) or weight.dtype != torch.float32:
             return F.hardtanh(super().forward(x), 0.0, self.clip)
+        bias = self._parameters.get("bias")
+        if bias is None:
+            bias = self.bias
         # The kernels update the running statistics and the counter of batches.
-        rm, rv, count = (self.running_mean, self.running_var, self.num_batches_tracked) if self.track_running_stats else (None, None, None)
-        return _lib.ext().bn_clip(x, self.weight, self.bias, rm, rv, count, self.eps, self.momentum, self.clip)
+        b = self._buffers
+        rm, rv, count = (b["running_mean"], b["running_var"], b["num_batches_tracked"]) if self.track_running_stats else (None, None, None)
+        return _lib.ext().bn_clip(x, weight, bias, rm, rv, count, self.eps, self.momentum, self.clip)
 
     def extra_repr(self) -> str:
         return super().extra_repr() + f", clip={self.clip}"
