@@ -191,6 +191,12 @@ int bc_bn_clip_backward(const float* x, const float* dy, const float* gamma, con
                         const float* save_rstd, float* dx, float* dgamma, float* dbeta, double* acc, int N, int C, int HW,
                         float clip_hi, void* stream);
 
+/* CTC loss, mean over the batch, all utterances of T frames; csrc/cuda/ctc.h. */
+int bc_ctc_forward(const float* logp, const long long* labels, long long stride, const long long* lens, float* chains, float* nll, float* loss,
+                   int T, int B, int C, int Lmax, void* stream);
+int bc_ctc_backward(const float* logp, const long long* labels, long long stride, const long long* lens, const float* chains, const float* nll,
+                    const float* dloss, float* dlogp, int T, int B, int C, int Lmax, void* stream);
+
 /* Coordinator validation run on synthetic requests (unit tests). Returns the response type. */
 int bc_test_validate(int nranks, const int* ops, const int* dtypes, const int* devices, const int* ndims,
                      const long long* shapes, char* err_out, int err_cap, long long* dim0_out);

@@ -14,6 +14,7 @@
 
 #include "cuda/comm.h"
 #include "cuda/bn_clip.h"
+#include "cuda/ctc.h"
 #include "cuda/conv_rows.h"
 #include "cuda/gru_persistent.h"
 #include "runtime/runtime.h"
@@ -642,6 +643,24 @@ int bc_bn_clip_backward(const float* x, const float* dy, const float* gamma, con
   API_BEGIN
   check_cuda(gpu::bn_clip_backward(x, dy, gamma, beta, save_mean, save_rstd, dx, dgamma, dbeta, acc, N, C, HW, clip_hi,
                                    (cudaStream_t)stream), "batch-norm + clip backward launch");
+  return 0;
+  API_END(-1)
+}
+
+// ---- CTC loss (kernels in cuda/ctc.cu) -----------------------------------------------------------------
+
+int bc_ctc_forward(const float* logp, const long long* labels, long long stride, const long long* lens, float* chains, float* nll, float* loss,
+                   int T, int B, int C, int Lmax, void* stream) {
+  API_BEGIN
+  check_cuda(gpu::ctc_forward(logp, labels, stride, lens, chains, nll, loss, T, B, C, Lmax, (cudaStream_t)stream), "CTC loss launch");
+  return 0;
+  API_END(-1)
+}
+
+int bc_ctc_backward(const float* logp, const long long* labels, long long stride, const long long* lens, const float* chains, const float* nll,
+                    const float* dloss, float* dlogp, int T, int B, int C, int Lmax, void* stream) {
+  API_BEGIN
+  check_cuda(gpu::ctc_backward(logp, labels, stride, lens, chains, nll, dloss, dlogp, T, B, C, Lmax, (cudaStream_t)stream), "CTC gradient launch");
   return 0;
   API_END(-1)
 }

@@ -305,6 +305,48 @@ Tensor conv_rows(const Tensor& x, const Tensor& w, int64_t ph, int64_t pw) {
   return ConvRows::apply(x, w, ph, pw);
 }
 
+// ---- CTC loss -----------------------------------------------------------------------------------
+
+std::atomic<long long> g_ctc_launches{0};
+
+const long long* longs(const Tensor& t) { return reinterpret_cast<const long long*>(t.data_ptr<int64_t>()); }
+
+struct CtcMean : torch::autograd::Function<CtcMean> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& logp, const Tensor& labels, const Tensor& lens) {
+    const c10::cuda::CUDAGuard guard(logp.device());
+    const int64_t t = logp.size(0), b = logp.size(1), c = logp.size(2), l = labels.size(1), chains = 2 * b * t * (2 * l + 1);
+    Tensor work = at::empty({chains + b}, logp.options()), loss = at::empty({}, logp.options());
+    check(bc_ctc_forward(ptr(logp), longs(labels), l, longs(lens), ptr(work), ptr(work) + chains, ptr(loss), (int)t, (int)b, (int)c, (int)l,
+                         stream_of(logp)),
+          "bc_ctc_forward");
+    g_ctc_launches++;
+    ctx->save_for_backward({logp, labels, lens, work});
+    return loss;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &logp = saved[0], &labels = saved[1], &lens = saved[2], &work = saved[3];
+    const c10::cuda::CUDAGuard guard(logp.device());
+    const int64_t t = logp.size(0), b = logp.size(1), c = logp.size(2), l = labels.size(1), chains = 2 * b * t * (2 * l + 1);
+    const Tensor dloss = grads[0].contiguous();
+    Tensor dlogp = at::empty_like(logp);
+    check(bc_ctc_backward(ptr(logp), longs(labels), l, longs(lens), ptr(work), ptr(work) + chains, ptr(dloss), ptr(dlogp), (int)t, (int)b, (int)c,
+                          (int)l, stream_of(logp)),
+          "bc_ctc_backward");
+    g_ctc_launches++;
+    return {dlogp, Tensor(), Tensor()};
+  }
+};
+
+Tensor ctc_mean(const Tensor& logp, const Tensor& labels, const Tensor& lens) {
+  TORCH_CHECK(logp.is_cuda() && logp.scalar_type() == at::kFloat && logp.dim() == 3 && logp.numel() > 0 && labels.device() == logp.device() &&
+                  labels.scalar_type() == at::kLong && labels.dim() == 2 && labels.size(0) == logp.size(1) && lens.device() == logp.device() &&
+                  lens.scalar_type() == at::kLong && lens.dim() == 1 && lens.size(0) == logp.size(1),
+              "ctc_mean takes fp32 CUDA log-probabilities [T, B, C], labels [B, L] and lengths [B] on the same device");
+  return CtcMean::apply(logp.contiguous(), labels.contiguous(), lens.contiguous());
+}
+
 // ---- collectives of a group of one --------------------------------------------------------------
 
 int dtype_code(at::ScalarType t) {
@@ -347,5 +389,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("conv_supported", &conv_supported);
   m.def("conv_rows", &conv_rows);
   m.def("conv_launches", [] { return g_conv_launches.load(); });
+  m.def("ctc_mean", &ctc_mean);
+  m.def("ctc_launches", [] { return g_ctc_launches.load(); });
   m.def("allreduce_alone", &allreduce_alone);
 }

@@ -90,10 +90,10 @@ class DeepSpeech2(nn.Module):
         return F.log_softmax(self.fc(x), dim=-1)
 
     def loss(self, spect: torch.Tensor, labels: torch.Tensor, label_lengths: torch.Tensor) -> torch.Tensor:
-        logp = self.forward(spect)
-        t, b, _ = logp.shape
-        in_len = torch.full((b,), t, dtype=torch.long, device=logp.device)
-        return F.ctc_loss(logp, labels, in_len, label_lengths, blank=0, reduction="mean", zero_infinity=True)
+        from ..ops import ctc
+
+        lengths = ctc.Lengths(label_lengths)
+        return ctc.mean_loss(self.forward(spect), labels, lengths)
 
 
 def synthetic_batch(cfg: DS2Config, batch: int, device, generator=None, pin: bool = False):
