@@ -4,8 +4,8 @@ Two 2-D convolutions over (frequency, time) with batch norm and clipped ReLU, a 
 bidirectional GRU layers, a linear layer to the character classes and CTC loss. The reference
 ships no such model; its pieces there are Conv2D/cuDNN, FusedBatchNorm, Relu6-style clipping,
 GRU cells (tensorflow/contrib/rnn/kernels/gru_ops.h:69-119) or CudnnRNN, and a CPU-only CTC loss
-(tensorflow/core/kernels/ctc_loss_op.cc:167). Here the output layer and the loss are plain torch.nn
-modules on cuBLAS; the convolutions run on the library's tcgen05 kernels where these cover them
+(tensorflow/core/kernels/ctc_loss_op.cc:167). Here the output layer is a plain torch.nn module on
+cuBLAS; the loss is the library's on a GPU (`ops/ctc.py`); the convolutions run on the library's tcgen05 kernels where these cover them
 (`ops/conv_rows.py`, else cuDNN); batch norm and the clipped ReLU behind it are one
 module on the library's two-pass kernels (`ops/bn_clip.py`); the GRU stack keeps its `nn.GRU` module
 and parameters but, on a GPU that supports them, is evaluated by the library's persistent

@@ -28,7 +28,13 @@ def test_matches_ctc_loss(t, b, c, longest):
     want = F.ctc_loss(F.log_softmax(xd, -1), labels.cpu(), torch.full((b,), t), lens.cpu(), blank=0, reduction="mean", zero_infinity=True)
     (wgrad,) = torch.autograd.grad(want * 3, xd)
     assert abs(loss.item() - want.item()) <= 1e-5 * abs(want.item()) + 1e-6
-    assert (grad.cpu().double() - wgrad).norm().item() <= 2e-4 * wgrad.norm().item() + 1e-7
+    # Sums of t logarithms in fp32 round the more, the longer they are: torch's own fp32 gradient is the measure.
+    xt = x.detach().requires_grad_(True)
+    theirs = F.ctc_loss(F.log_softmax(xt, -1), labels, torch.full((b,), t), lens, blank=0, reduction="mean", zero_infinity=True)
+    (tgrad,) = torch.autograd.grad(theirs * 3, xt)
+    mine, torchs = [(g.cpu().double() - wgrad).norm().item() / (wgrad.norm().item() + 1e-9) for g in (grad, tgrad)]
+    print(f"relative error {mine:.2e}, torch {torchs:.2e}")
+    assert mine <= 1.2 * torchs + 5e-6
 
 
 def test_wrong_lengths_are_refused():
