@@ -197,6 +197,10 @@ int bc_ctc_forward(const float* logp, const long long* labels, long long stride,
 int bc_ctc_backward(const float* logp, const long long* labels, long long stride, const long long* lens, const float* chains, const float* nll,
                     const float* dloss, float* dlogp, int T, int B, int C, int Lmax, void* stream);
 
+/* out[b][c][r] = in[b][r][c], fp32; csrc/cuda/transpose.h. */
+int bc_transpose(const float* in, float* out, int batch, int rows, int cols, long long in_row, long long in_batch, long long out_row,
+                 long long out_batch, void* stream);
+
 /* Coordinator validation run on synthetic requests (unit tests). Returns the response type. */
 int bc_test_validate(int nranks, const int* ops, const int* dtypes, const int* devices, const int* ndims,
                      const long long* shapes, char* err_out, int err_cap, long long* dim0_out);

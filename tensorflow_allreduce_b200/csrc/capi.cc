@@ -15,6 +15,7 @@
 #include "cuda/comm.h"
 #include "cuda/bn_clip.h"
 #include "cuda/ctc.h"
+#include "cuda/transpose.h"
 #include "cuda/conv_rows.h"
 #include "cuda/gru_persistent.h"
 #include "runtime/runtime.h"
@@ -661,6 +662,14 @@ int bc_ctc_backward(const float* logp, const long long* labels, long long stride
                     const float* dloss, float* dlogp, int T, int B, int C, int Lmax, void* stream) {
   API_BEGIN
   check_cuda(gpu::ctc_backward(logp, labels, stride, lens, chains, nll, dloss, dlogp, T, B, C, Lmax, (cudaStream_t)stream), "CTC gradient launch");
+  return 0;
+  API_END(-1)
+}
+
+int bc_transpose(const float* in, float* out, int batch, int rows, int cols, long long in_row, long long in_batch, long long out_row,
+                 long long out_batch, void* stream) {
+  API_BEGIN
+  check_cuda(gpu::transpose(in, out, batch, rows, cols, in_row, in_batch, out_row, out_batch, (cudaStream_t)stream), "transposition launch");
   return 0;
   API_END(-1)
 }

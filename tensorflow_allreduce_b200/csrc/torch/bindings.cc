@@ -347,6 +347,35 @@ Tensor ctc_mean(const Tensor& logp, const Tensor& labels, const Tensor& lens) {
   return CtcMean::apply(logp.contiguous(), labels.contiguous(), lens.contiguous());
 }
 
+// ---- activations of a convolution, time first ---------------------------------------------------
+
+// [B, ..., T] -> [T, B, features] of contiguous fp32 activations.
+struct TimeMajor : torch::autograd::Function<TimeMajor> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t b = x.size(0), t = x.size(-1), k = x.numel() / (b * t);
+    ctx->saved_data["shape"] = x.sizes().vec();
+    Tensor y = at::empty({t, b, k}, x.options());
+    check(bc_transpose(ptr(x), ptr(y), (int)b, (int)k, (int)t, t, k * t, b * k, k, stream_of(x)), "bc_transpose");
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor dy = grads[0].contiguous();
+    const c10::cuda::CUDAGuard guard(dy.device());
+    const int64_t t = dy.size(0), b = dy.size(1), k = dy.size(2);
+    Tensor dx = at::empty(ctx->saved_data["shape"].toIntVector(), dy.options());
+    check(bc_transpose(ptr(dy), ptr(dx), (int)b, (int)t, (int)k, b * k, k, t, k * t, stream_of(dy)), "bc_transpose");
+    return {dx};
+  }
+};
+
+Tensor time_major(const Tensor& x) {
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 2 && x.numel() > 0 && x.size(0) <= 65535,
+              "time_major takes contiguous fp32 CUDA activations");
+  return TimeMajor::apply(x);
+}
+
 // ---- collectives of a group of one --------------------------------------------------------------
 
 int dtype_code(at::ScalarType t) {
@@ -391,5 +420,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("conv_launches", [] { return g_conv_launches.load(); });
   m.def("ctc_mean", &ctc_mean);
   m.def("ctc_launches", [] { return g_ctc_launches.load(); });
+  m.def("time_major", &time_major);
   m.def("allreduce_alone", &allreduce_alone);
 }

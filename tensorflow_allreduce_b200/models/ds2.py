@@ -80,7 +80,12 @@ class DeepSpeech2(nn.Module):
         [frames', batch, classes]."""
         x = self.conv(spect.unsqueeze(1))                 # [B, C, F', T']
         b, c, f, t = x.shape
-        x = x.view(b, c * f, t).permute(2, 0, 1).contiguous()   # [T', B, C*F']
+        if x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and 0 < x.numel() and b <= 65535:
+            from .. import _lib
+
+            x = _lib.ext().time_major(x)                  # [T', B, C*F']
+        else:
+            x = x.view(b, c * f, t).permute(2, 0, 1).contiguous()
         if self._use_persistent(x):
             from ..ops import persistent_gru
 
