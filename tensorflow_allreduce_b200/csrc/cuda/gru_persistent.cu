@@ -475,7 +475,13 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     // loads of this thread: K tiles kt0, kt0 + kTilesPerLoad, ... below ntile, the last one only if it has these chunks
     const int tiles_mine = chunk < last_chunks ? pl.ntile : pl.ntile - 1;
     const int mine = b < B && kt0 < tiles_mine ? (tiles_mine - kt0 + kTilesPerLoad - 1) / kTilesPerLoad : 0;
-    const uint32_t pause = (uint32_t)(pl.ntile * B * 128) / 80;      // cycles
+    // Cycles from a block's own publication to its first poll: about what the operand words of a step take to arrive, but
+    // not so little that polls meet the partial sums of groups that are still exchanging them, and not so much that this block is the
+    // last one. Measured at 15 shapes for 55 to 160 bytes per cycle; nothing to exchange: C = 1. Against `read` alone, us per
+    // step: forward H = 1024 B = 32 3.86 -> 3.78, B = 8 2.92 -> 2.79, B = 1 2.93 -> 2.59; H = 256 B = 32 2.30 -> 2.20; both passes
+    // H = 1024 B = 1 5.95 -> 5.34; none of the 15 slower by more than 0.7 %.
+    const uint32_t read = (uint32_t)(pl.ntile * B * 128) / 80;
+    const uint32_t pause = C == 1 ? read / 2 : C == 2 ? min(max(read, 300u), 600u) : C == 4 ? min(read, 300u) : max(read, (uint32_t)p.d.H / 3);
     constexpr int kSpan = kLoadsPerGroup == 4 ? 1 : 3;           // groups whose loads are in flight together
     bool good = true;
     // Every step is gone through to the end even when a wait has run out (the waits then end at once): the gate warps count
