@@ -258,7 +258,7 @@ struct ConvRows : torch::autograd::Function<ConvRows> {
     Tensor y = at::empty({x.size(0), 32, c.Ho(), c.Wo()}, x.options());
     check(bc_conv_forward(c.v, ptr(x), ptr(wc), ptr(y), scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, stream_of(x)), "bc_conv_forward");
     g_conv_launches++;
-    ctx->save_for_backward({x, wc});
+    ctx->save_for_backward({x, w});
     ctx->saved_data["ph"] = ph;
     ctx->saved_data["pw"] = pw;
     return y;
@@ -266,11 +266,18 @@ struct ConvRows : torch::autograd::Function<ConvRows> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w = saved[1];
+    const Tensor& x = saved[0];
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t ph = ctx->saved_data["ph"].toInt(), pw = ctx->saved_data["pw"].toInt();
-    const Conv c(x, w, ph, pw);
-    const Tensor dy = grads[0].contiguous(), scratch = c.scratch(x);
+    const Conv c(x, saved[1], ph, pw);
+    auto by_torch = [&](bool need_x, bool need_w) {
+      return at::convolution_backward(grads[0], x, saved[1], c10::nullopt, {2, c.v[8]}, {ph, pw}, {1, 1}, false, {0, 0}, 1, {need_x, need_w, false});
+    };
+    if (at::GradMode::is_enabled()) {      // the gradients are to be differentiated again
+      const auto d = by_torch(ctx->needs_input_grad(0), ctx->needs_input_grad(1));
+      return {std::get<0>(d), std::get<1>(d), Tensor(), Tensor()};
+    }
+    const Tensor w = saved[1].contiguous(), dy = grads[0].contiguous(), scratch = c.scratch(x);
     unsigned* status = (unsigned*)gru_status(x);
     Tensor dx, dw;
     if (ctx->needs_input_grad(1)) {
@@ -284,8 +291,7 @@ struct ConvRows : torch::autograd::Function<ConvRows> {
         check(bc_conv_backward_input(c.v, ptr(dy), ptr(w), ptr(dx), scratch.data_ptr(), status, g_gru_timeout_s, stream_of(x)), "bc_conv_backward_input");
         g_conv_launches++;
       } else {       // the spectrogram's gradient is not part of training
-        const int64_t sw = c.v[8];
-        dx = std::get<0>(at::convolution_backward(dy, x, w, c10::nullopt, {2, sw}, {ph, pw}, {1, 1}, false, {0, 0}, 1, {true, false, false}));
+        dx = std::get<0>(by_torch(true, false));
       }
     }
     return {dx, dw, Tensor(), Tensor()};

@@ -1,0 +1,40 @@
+"""The native call paths under everything that a torch operator supports and a raw kernel does not see."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _conv(cin=32):
+    from tensorflow_allreduce_b200.ops import conv_rows
+
+    torch.manual_seed(cin)
+    m = conv_rows.RowConv2d(cin, 32, (5, 3), stride=(2, 1 if cin == 32 else 2), padding=(2, 1), bias=False).cuda()
+    return m, torch.randn(2, cin, 17, 40, device="cuda", requires_grad=True)
+
+
+def _stock(m, x, w):
+    return F.conv2d(x, w, None, m.stride, m.padding)
+
+
+def _close(got, want, rel=2e-3):
+    assert (got.double() - want).norm().item() <= rel * want.norm().item() + 1e-9
+
+
+@pytest.mark.parametrize("cin", [1, 32])
+@pytest.mark.parametrize("strided_weight", [False, True])
+def test_second_derivatives_of_a_convolution(cin, strided_weight):
+    m, x = _conv(cin)
+    if strided_weight:
+        m.weight = torch.nn.Parameter(m.weight.detach().permute(3, 2, 1, 0).contiguous().permute(3, 2, 1, 0))
+    g = torch.randn_like(m(x)).requires_grad_(True)
+
+    def second(y, x, w, g):
+        gx, gw = torch.autograd.grad(y, [x, w], g, create_graph=True)
+        return [gx, gw, *torch.autograd.grad((gx ** 3).sum() + (gw ** 2).sum(), [x, w, g])]
+
+    got = second(m(x), x, m.weight, g)
+    xd, wd, gd = [t.detach().double().requires_grad_(True) for t in (x, m.weight, g)]
+    for a, b in zip(got, second(_stock(m, xd, wd), xd, wd, gd)):
+        _close(a, b)
