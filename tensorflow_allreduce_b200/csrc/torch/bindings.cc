@@ -367,6 +367,8 @@ struct TimeMajor : torch::autograd::Function<TimeMajor> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (at::GradMode::is_enabled())        // the gradient is to be differentiated again
+      return {grads[0].permute({1, 2, 0}).reshape(ctx->saved_data["shape"].toIntVector())};
     const Tensor dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());
     const int64_t t = dy.size(0), b = dy.size(1), k = dy.size(2);

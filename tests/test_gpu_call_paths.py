@@ -38,3 +38,16 @@ def test_second_derivatives_of_a_convolution(cin, strided_weight):
     xd, wd, gd = [t.detach().double().requires_grad_(True) for t in (x, m.weight, g)]
     for a, b in zip(got, second(_stock(m, xd, wd), xd, wd, gd)):
         _close(a, b)
+
+
+def test_second_derivatives_of_the_time_first_order():
+    from tensorflow_allreduce_b200 import _lib
+
+    x = torch.randn(3, 4, 5, 70, device="cuda", requires_grad=True)
+    y = _lib.ext().time_major(x)
+    g = torch.randn_like(y).requires_grad_(True)
+    (gx,) = torch.autograd.grad(y, x, g, create_graph=True)
+    assert torch.equal(gx, g.permute(1, 2, 0).reshape(x.shape))
+    v = torch.randn_like(gx)
+    (gg,) = torch.autograd.grad((gx * v).sum(), g)
+    assert torch.equal(gg, v.reshape(3, 20, 70).permute(2, 0, 1))
