@@ -8,6 +8,8 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 
 #include <atomic>
 #include <map>
@@ -341,6 +343,9 @@ struct CtcMean : torch::autograd::Function<CtcMean> {
                           (int)l, stream_of(logp)),
           "bc_ctc_backward");
     g_ctc_launches++;
+    if (at::GradMode::is_enabled())        // there is no second derivative, in torch's loss either: asking for it is an error
+      torch::autograd::set_history(dlogp, std::make_shared<torch::autograd::Error>("the CTC loss cannot be differentiated twice",
+                                                                                  torch::autograd::collect_next_edges(logp, grads[0])));
     return {dlogp, Tensor(), Tensor()};
   }
 };

@@ -51,3 +51,20 @@ def test_second_derivatives_of_the_time_first_order():
     v = torch.randn_like(gx)
     (gg,) = torch.autograd.grad((gx * v).sum(), g)
     assert torch.equal(gg, v.reshape(3, 20, 70).permute(2, 0, 1))
+
+
+def test_second_derivative_of_the_loss_is_refused():
+    from tensorflow_allreduce_b200.ops import ctc
+
+    x = torch.randn(20, 2, 5, device="cuda", requires_grad=True)
+    labels, lens = torch.randint(1, 5, (2, 4), device="cuda"), torch.tensor([4, 2], device="cuda")
+    for mine in (False, True):
+        logp = F.log_softmax(x, -1)
+        loss = (ctc.mean_loss(logp, labels, ctc.Lengths(lens)) if mine else
+                F.ctc_loss(logp, labels, torch.full((2,), 20), lens, blank=0, reduction="mean", zero_infinity=True))
+        (g,) = torch.autograd.grad(loss * 3, x, create_graph=True)
+        if not mine:
+            first = g.detach()
+        torch.testing.assert_close(g.detach(), first, rtol=1e-4, atol=1e-6)
+        with pytest.raises(RuntimeError):
+            torch.autograd.grad(g.square().sum(), x)
