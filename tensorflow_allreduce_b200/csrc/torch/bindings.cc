@@ -10,6 +10,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
 #include <map>
@@ -31,6 +32,10 @@ void check(int rc, const char* what) {
 
 float* ptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
 void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// May the kernels be called as they are? Not under something that follows torch's operators: it does not see them, and a trace
+// would hold this call's values as constants.
+bool plain(const Tensor&) { return !torch::jit::tracer::isTracing(); }
 
 // ---- batch norm + clipped ReLU -----------------------------------------------------------------
 
@@ -80,6 +85,10 @@ Tensor bn_clip(const Tensor& x, const Tensor& weight, const Tensor& bias, const 
                const c10::optional<Tensor>& running_var, const c10::optional<Tensor>& batches, double eps, double momentum, double clip) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 2 && x.numel() > 0,
               "bn_clip needs a contiguous fp32 CUDA tensor");
+  if (!plain(x)) {
+    if (batches) Tensor(*batches).add_(1);
+    return at::hardtanh(at::batch_norm(x, weight, bias, running_mean, running_var, true, momentum, eps, at::globalContext().userEnabledCuDNN()), 0.0, clip);
+  }
   return BnClip::apply(x, weight, bias, running_mean, running_var, batches, eps, momentum, clip);
 }
 
@@ -302,7 +311,7 @@ struct ConvRows : torch::autograd::Function<ConvRows> {
 
 bool conv_supported(const Tensor& x, const Tensor& w, int64_t ph, int64_t pw) {
   if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != at::kFloat || w.scalar_type() != at::kFloat || x.dim() != 4 || w.dim() != 4 ||
-      !x.is_contiguous() || w.size(0) != 32 || w.size(1) != x.size(1) || x.size(0) > 65535)
+      !x.is_contiguous() || w.size(0) != 32 || w.size(1) != x.size(1) || x.size(0) > 65535 || !plain(x))
     return false;
   const Conv c(x, w, ph, pw);
   return bc_conv_supported(x.device().index(), c.v) == 1;
@@ -386,6 +395,7 @@ struct TimeMajor : torch::autograd::Function<TimeMajor> {
 Tensor time_major(const Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 2 && x.numel() > 0 && x.size(0) <= 65535,
               "time_major takes contiguous fp32 CUDA activations");
+  if (!plain(x)) return x.flatten(1, -2).permute({2, 0, 1}).contiguous();
   return TimeMajor::apply(x);
 }
 
@@ -421,6 +431,7 @@ c10::optional<Tensor> allreduce_alone(const std::string& name, const Tensor& ten
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("plain", &plain);
   m.def("bn_clip", &bn_clip);
   m.def("bn_launches", [] { return g_bn_launches.load(); });
   m.def("gru_stack", &gru_stack);

@@ -28,7 +28,7 @@ class Lengths:
         self.device = lengths
         self.event = None
         self.host = lengths
-        if lengths.is_cuda:
+        if lengths.is_cuda and _lib.ext().plain(lengths):
             with torch.cuda.device(lengths.device):
                 self.host = torch.empty(lengths.shape, dtype=lengths.dtype, pin_memory=True)
                 self.host.copy_(lengths, non_blocking=True)
@@ -47,7 +47,7 @@ def mean_loss(logp: torch.Tensor, labels: torch.Tensor, lengths: Lengths) -> tor
     """logp: [T, B, C] log-probabilities out of a softmax; labels: [B, L]; class 0 is the blank."""
     t, b, _ = logp.shape
     n = lengths.device
-    if (logp.is_cuda and logp.dtype == torch.float32 and logp.numel() > 0 and labels.dim() == 2 and labels.dtype == torch.int64
+    if (logp.is_cuda and _lib.ext().plain(logp) and logp.dtype == torch.float32 and logp.numel() > 0 and labels.dim() == 2 and labels.dtype == torch.int64
             and labels.device == logp.device and labels.shape[0] == b <= 65535 and labels.shape[1] <= 511
             and n.dtype == torch.int64 and tuple(n.shape) == (b,)):
         lengths.check(labels.shape[1])

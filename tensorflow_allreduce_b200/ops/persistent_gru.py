@@ -61,10 +61,18 @@ def supported(T: int, B: int, H: int, ndir: int, device=None) -> bool:
     return _lib.lib().bc_gru_supported(idx, int(T), int(B), int(H), int(ndir)) == 1
 
 
+def _stack(x: torch.Tensor, weights: List[torch.Tensor], layers: int) -> torch.Tensor:
+    if torch._C._get_tracing_state() is not None:      # a trace does not see the kernels: it holds torch's operator
+        nd = len(weights) // (4 * layers)
+        h = torch.zeros(layers * nd, x.shape[1], weights[1].shape[1], device=x.device)
+        return torch._VF.gru(x, h, weights, True, layers, 0.0, True, nd == 2, False)[0]
+    return _ext().gru_stack(x, weights, layers)
+
+
 def gru_layer(x: torch.Tensor, w_ih: torch.Tensor, w_hh: torch.Tensor, b_ih: torch.Tensor, b_hh: torch.Tensor) -> torch.Tensor:
     """One GRU layer over a time-major fp32 sequence x [T, B, I] with zero initial state.
     Parameters are stacked over the directions (1 or 2). Returns [T, B, ndir * H]."""
-    return _ext().gru_stack(x, [t[d] for d in range(w_hh.shape[0]) for t in (w_ih, w_hh, b_ih, b_hh)], 1)
+    return _stack(x, [t[d] for d in range(w_hh.shape[0]) for t in (w_ih, w_hh, b_ih, b_hh)], 1)
 
 
 def gru_forward(rnn: torch.nn.GRU, x: torch.Tensor) -> torch.Tensor:
@@ -77,4 +85,4 @@ def gru_forward(rnn: torch.nn.GRU, x: torch.Tensor) -> torch.Tensor:
     for layer in range(rnn.num_layers):
         for sfx in (f"_l{layer}", f"_l{layer}_reverse")[:nd]:
             weights += (getattr(rnn, "weight_ih" + sfx), getattr(rnn, "weight_hh" + sfx), getattr(rnn, "bias_ih" + sfx), getattr(rnn, "bias_hh" + sfx))
-    return _ext().gru_stack(x, weights, rnn.num_layers)
+    return _stack(x, weights, rnn.num_layers)

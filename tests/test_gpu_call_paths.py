@@ -68,3 +68,78 @@ def test_second_derivative_of_the_loss_is_refused():
         torch.testing.assert_close(g.detach(), first, rtol=1e-4, atol=1e-6)
         with pytest.raises(RuntimeError):
             torch.autograd.grad(g.square().sum(), x)
+
+
+@pytest.mark.parametrize("cin", [1, 32])
+def test_traced_convolution(cin):
+    m, x = _conv(cin)
+    with torch.no_grad():
+        traced = torch.jit.trace(m, (x,))
+        other = torch.randn(3, cin, 23, 50, device="cuda")
+        _close(traced(other), _stock(m, other.double(), m.weight.double()))
+
+
+def test_traced_time_first_order():
+    from tensorflow_allreduce_b200 import _lib
+
+    traced = torch.jit.trace(lambda x: _lib.ext().time_major(x), (torch.randn(2, 3, 5, 7, device="cuda"),), check_trace=False)
+    x = torch.randn(2, 3, 5, 7, device="cuda")
+    assert torch.equal(traced(x), x.reshape(2, 15, 7).permute(2, 0, 1))
+
+
+def test_traced_loss():
+    from tensorflow_allreduce_b200.ops import ctc
+
+    labels, lens = torch.randint(1, 5, (2, 4), device="cuda"), torch.tensor([4, 2], device="cuda")
+
+    def loss(x):
+        return ctc.mean_loss(F.log_softmax(x, -1), labels, ctc.Lengths(lens))
+
+    traced = torch.jit.trace(loss, (torch.randn(20, 2, 5, device="cuda"),), check_trace=False)
+    x = torch.randn(20, 2, 5, device="cuda")
+    torch.testing.assert_close(traced(x), loss(x))
+
+
+@pytest.mark.parametrize("layers,nd", [(1, 1), (2, 2)])
+def test_traced_gru(layers, nd):
+    from tensorflow_allreduce_b200.ops import persistent_gru as pg
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.rnn = torch.nn.GRU(40, 128, num_layers=layers, bidirectional=nd == 2)
+
+        def forward(self, x):
+            return pg.gru_forward(self.rnn, x)
+
+    torch.manual_seed(layers)
+    net = Net().cuda().eval()
+    traced = torch.jit.trace(net, (torch.randn(6, 3, 40, device="cuda"),), check_trace=False)
+    x = torch.randn(9, 2, 40, device="cuda", requires_grad=True)
+    want = net(x)
+    before = pg.launch_count
+    y = traced(x)
+    assert pg.launch_count == before
+    _close(y, want.double())
+    for a, b in zip(torch.autograd.grad(y.sum(), [x, *net.parameters()]), torch.autograd.grad(want.sum(), [x, *net.parameters()])):
+        _close(a, b.double(), 5e-3)
+
+
+def test_traced_norm():
+    from tensorflow_allreduce_b200.ops import bn_clip
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.a, self.b = bn_clip.BatchNormClip2d(4), bn_clip.BatchNormClip2d(4, clip=1.0)
+
+        def forward(self, x):
+            return self.a(x), bn_clip.bn_clip(x, self.b.weight, self.b.bias, None, None, 1e-5, 0.1, 1.0)
+
+    net = Net().cuda()
+    traced = torch.jit.trace(net, (torch.randn(3, 4, 5, 6, device="cuda"),), check_trace=False)
+    x = torch.randn(2, 4, 7, 6, device="cuda")
+    count = net.a.num_batches_tracked.item()
+    for a, b in zip(traced(x), net(x)):
+        torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
+    assert net.a.num_batches_tracked.item() == count + 2
