@@ -7,6 +7,7 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -33,9 +34,16 @@ void check(int rc, const char* what) {
 float* ptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
 void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
-// May the kernels be called as they are? Not under something that follows torch's operators: it does not see them, and a trace
-// would hold this call's values as constants.
-bool plain(const Tensor&) { return !torch::jit::tracer::isTracing(); }
+// Something that follows torch's operators does not see the kernels: a trace would hold this call's values as constants,
+// forward-mode derivatives would stop here, the batches and gradients of torch.func and tensors without storage have no memory to
+// hand to them.
+bool traced() { return torch::jit::tracer::isTracing(); }
+bool has_tangent(const Tensor& t) { return torch::autograd::isFwGradDefined(t); }
+bool plain(const Tensor& t) {
+  constexpr c10::DispatchKeySet wrappers({c10::DispatchKey::Batched, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                          c10::DispatchKey::Functionalize, c10::DispatchKey::Python});
+  return !traced() && !c10::impl::TorchDispatchModeTLS::any_modes_set() && !t.key_set().has_any(wrappers) && !has_tangent(t);
+}
 
 // ---- batch norm + clipped ReLU -----------------------------------------------------------------
 
@@ -85,7 +93,7 @@ Tensor bn_clip(const Tensor& x, const Tensor& weight, const Tensor& bias, const 
                const c10::optional<Tensor>& running_var, const c10::optional<Tensor>& batches, double eps, double momentum, double clip) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 2 && x.numel() > 0,
               "bn_clip needs a contiguous fp32 CUDA tensor");
-  if (!plain(x)) {
+  if (traced()) {
     if (batches) Tensor(*batches).add_(1);
     return at::hardtanh(at::batch_norm(x, weight, bias, running_mean, running_var, true, momentum, eps, at::globalContext().userEnabledCuDNN()), 0.0, clip);
   }
@@ -211,7 +219,12 @@ Tensor gru_stack(Tensor x, const std::vector<Tensor>& weights, int64_t layers) {
   for (int64_t l = 0; l < layers; l++) {
     const at::TensorList w(weights.data() + l * per, per);
     bool grad = at::GradMode::is_enabled() && x.requires_grad();
-    for (const Tensor& t : w) grad = grad || (at::GradMode::is_enabled() && t.requires_grad());
+    bool tangent = has_tangent(x);
+    for (const Tensor& t : w) {
+      grad = grad || (at::GradMode::is_enabled() && t.requires_grad());
+      tangent = tangent || has_tangent(t);
+    }
+    TORCH_CHECK(!tangent, "the persistent GRU kernels have no forward-mode derivative");
     if (grad) {
       x = GruLayer::apply(x, w);
     } else {
@@ -284,7 +297,7 @@ struct ConvRows : torch::autograd::Function<ConvRows> {
     auto by_torch = [&](bool need_x, bool need_w) {
       return at::convolution_backward(grads[0], x, saved[1], c10::nullopt, {2, c.v[8]}, {ph, pw}, {1, 1}, false, {0, 0}, 1, {need_x, need_w, false});
     };
-    if (at::GradMode::is_enabled()) {      // the gradients are to be differentiated again
+    if (at::GradMode::is_enabled() || !plain(grads[0])) {      // the gradients are to be differentiated again, or are many
       const auto d = by_torch(ctx->needs_input_grad(0), ctx->needs_input_grad(1));
       return {std::get<0>(d), std::get<1>(d), Tensor(), Tensor()};
     }
@@ -311,7 +324,7 @@ struct ConvRows : torch::autograd::Function<ConvRows> {
 
 bool conv_supported(const Tensor& x, const Tensor& w, int64_t ph, int64_t pw) {
   if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != at::kFloat || w.scalar_type() != at::kFloat || x.dim() != 4 || w.dim() != 4 ||
-      !x.is_contiguous() || w.size(0) != 32 || w.size(1) != x.size(1) || x.size(0) > 65535 || !plain(x))
+      !x.is_contiguous() || w.size(0) != 32 || w.size(1) != x.size(1) || x.size(0) > 65535 || !plain(x) || !plain(w))
     return false;
   const Conv c(x, w, ph, pw);
   return bc_conv_supported(x.device().index(), c.v) == 1;
@@ -346,7 +359,8 @@ struct CtcMean : torch::autograd::Function<CtcMean> {
     const Tensor &logp = saved[0], &labels = saved[1], &lens = saved[2], &work = saved[3];
     const c10::cuda::CUDAGuard guard(logp.device());
     const int64_t t = logp.size(0), b = logp.size(1), c = logp.size(2), l = labels.size(1), chains = 2 * b * t * (2 * l + 1);
-    const Tensor dloss = grads[0].contiguous();
+    const bool one = plain(grads[0]);          // else a batch of them
+    const Tensor dloss = one ? grads[0].contiguous() : at::ones({}, logp.options());
     Tensor dlogp = at::empty_like(logp);
     check(bc_ctc_backward(ptr(logp), longs(labels), l, longs(lens), ptr(work), ptr(work) + chains, ptr(dloss), ptr(dlogp), (int)t, (int)b, (int)c,
                           (int)l, stream_of(logp)),
@@ -355,7 +369,7 @@ struct CtcMean : torch::autograd::Function<CtcMean> {
     if (at::GradMode::is_enabled())        // there is no second derivative, in torch's loss either: asking for it is an error
       torch::autograd::set_history(dlogp, std::make_shared<torch::autograd::Error>("the CTC loss cannot be differentiated twice",
                                                                                   torch::autograd::collect_next_edges(logp, grads[0])));
-    return {dlogp, Tensor(), Tensor()};
+    return {one ? dlogp : dlogp * grads[0], Tensor(), Tensor()};
   }
 };
 
@@ -381,7 +395,7 @@ struct TimeMajor : torch::autograd::Function<TimeMajor> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    if (at::GradMode::is_enabled())        // the gradient is to be differentiated again
+    if (at::GradMode::is_enabled() || !plain(grads[0]))        // the gradient is to be differentiated again, or is many
       return {grads[0].permute({1, 2, 0}).reshape(ctx->saved_data["shape"].toIntVector())};
     const Tensor dy = grads[0].contiguous();
     const c10::cuda::CUDAGuard guard(dy.device());

@@ -49,7 +49,8 @@ def mean_loss(logp: torch.Tensor, labels: torch.Tensor, lengths: Lengths) -> tor
     n = lengths.device
     if (logp.is_cuda and _lib.ext().plain(logp) and logp.dtype == torch.float32 and logp.numel() > 0 and labels.dim() == 2 and labels.dtype == torch.int64
             and labels.device == logp.device and labels.shape[0] == b <= 65535 and labels.shape[1] <= 511
-            and n.dtype == torch.int64 and tuple(n.shape) == (b,)):
+            and n.dtype == torch.int64 and tuple(n.shape) == (b,)
+            and _lib.ext().plain(labels) and _lib.ext().plain(n)):
         lengths.check(labels.shape[1])
         return _lib.ext().ctc_mean(logp, labels, n.to(logp.device, non_blocking=True))
     in_len = torch.full((b,), t, dtype=torch.long, device=logp.device)

@@ -1,6 +1,7 @@
 """The native call paths under everything that a torch operator supports and a raw kernel does not see."""
 import pytest
 import torch
+import torch.autograd.forward_ad as fwd
 import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
@@ -143,3 +144,94 @@ def test_traced_norm():
     for a, b in zip(traced(x), net(x)):
         torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
     assert net.a.num_batches_tracked.item() == count + 2
+
+
+@pytest.mark.parametrize("cin", [1, 32])
+def test_forward_mode_through_a_convolution(cin):
+    m, x = _conv(cin)
+    t = torch.randn_like(x)
+    with fwd.dual_level():
+        y = fwd.unpack_dual(m(fwd.make_dual(x.detach(), t)))
+    _close(y.primal, _stock(m, x.detach().double(), m.weight.double()))
+    _close(y.tangent, _stock(m, t.double(), m.weight.double()))
+
+
+def test_forward_mode_through_the_time_first_order():
+    from tensorflow_allreduce_b200 import _lib
+
+    x, t = torch.randn(2, 3, 5, 7, device="cuda"), torch.randn(2, 3, 5, 7, device="cuda")
+    with fwd.dual_level():
+        y = fwd.unpack_dual(_lib.ext().time_major(fwd.make_dual(x, t)))
+    assert torch.equal(y.tangent, t.reshape(2, 15, 7).permute(2, 0, 1))
+
+
+def test_forward_mode_through_a_gru_is_refused():
+    from tensorflow_allreduce_b200.ops import persistent_gru as pg
+
+    rnn = torch.nn.GRU(40, 128).cuda()
+    x = torch.randn(6, 3, 40, device="cuda")
+    for p in rnn.parameters():
+        p.requires_grad_(False)
+    with fwd.dual_level():
+        with pytest.raises(RuntimeError):
+            pg.gru_forward(rnn, fwd.make_dual(x, torch.ones_like(x)))
+
+
+def test_forward_mode_through_a_norm_is_refused():
+    from tensorflow_allreduce_b200.ops import bn_clip
+
+    m = bn_clip.BatchNormClip2d(4).cuda()
+    x = torch.randn(3, 4, 5, 6, device="cuda")
+    with fwd.dual_level():
+        with pytest.raises(RuntimeError):
+            m(fwd.make_dual(x, torch.ones_like(x)))
+
+
+@pytest.mark.parametrize("cin", [1, 32])
+def test_batches_of_gradients_and_vmap(cin):
+    m, x = _conv(cin)
+    y = m(x)
+    g = torch.randn(3, *y.shape, device="cuda")
+    gx, gw = torch.autograd.grad(y, [x, m.weight], g, is_grads_batched=True)
+    for i in range(3):
+        xd, wd = x.detach().double().requires_grad_(True), m.weight.detach().double().requires_grad_(True)
+        wx, ww = torch.autograd.grad(_stock(m, xd, wd), [xd, wd], g[i].double())
+        _close(gx[i], wx)
+        _close(gw[i], ww)
+    xs = torch.randn(3, *x.shape, device="cuda")
+    with torch.no_grad():
+        _close(torch.vmap(m)(xs), torch.stack([_stock(m, v.double(), m.weight.double()) for v in xs]))
+    f = torch.func.grad(lambda w: torch.func.functional_call(m, {"weight": w}, (x.detach(),)).square().sum())
+    wd = m.weight.detach().double().requires_grad_(True)
+    _close(f(m.weight.detach()), torch.autograd.grad(_stock(m, x.detach().double(), wd).square().sum(), wd)[0])
+
+
+def test_batches_of_gradients_of_the_time_first_order_and_the_loss():
+    from tensorflow_allreduce_b200 import _lib
+    from tensorflow_allreduce_b200.ops import ctc
+
+    x = torch.randn(2, 3, 5, 7, device="cuda", requires_grad=True)
+    y = _lib.ext().time_major(x)
+    g = torch.randn(4, *y.shape, device="cuda")
+    (gx,) = torch.autograd.grad(y, x, g, is_grads_batched=True)
+    assert torch.equal(gx, torch.stack([v.permute(1, 2, 0).reshape(x.shape) for v in g]))
+    with torch.no_grad():
+        xs = torch.randn(4, 2, 3, 5, 7, device="cuda")
+        assert torch.equal(torch.vmap(lambda v: _lib.ext().time_major(v))(xs), torch.stack([v.reshape(2, 15, 7).permute(2, 0, 1) for v in xs]))
+    s = torch.randn(20, 2, 5, device="cuda", requires_grad=True)
+    labels, lens = torch.randint(1, 5, (2, 4), device="cuda"), torch.tensor([4, 2], device="cuda")
+    loss = ctc.mean_loss(F.log_softmax(s, -1), labels, ctc.Lengths(lens))
+    (one,) = torch.autograd.grad(loss, s, retain_graph=True)
+    (many,) = torch.autograd.grad(loss, s, torch.tensor([1.0, -2.0], device="cuda"), is_grads_batched=True)
+    torch.testing.assert_close(many, torch.stack([one, -2 * one]))
+
+
+def test_dispatch_modes_see_the_operators():
+    from torch.utils.flop_counter import FlopCounterMode
+
+    m, x = _conv()
+    with FlopCounterMode(display=False) as mine, torch.no_grad():
+        m(x)
+    with FlopCounterMode(display=False) as stock, torch.no_grad():
+        _stock(m, x, m.weight)
+    assert mine.get_total_flops() == stock.get_total_flops() > 0
