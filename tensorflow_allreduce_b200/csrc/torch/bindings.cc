@@ -322,9 +322,13 @@ struct ConvRows : torch::autograd::Function<ConvRows> {
   }
 };
 
+// The operands are TF32: not where fp32 convolutions are asked for, by the flag of all of cuDNN or by that of its convolutions, and not
+// where cuDNN is off, since torch's own convolutions are fp32.
+bool tf32_allowed() { return at::globalContext().userEnabledCuDNN() && at::globalContext().allowTF32CuDNN(at::Float32Op::CONV); }
+
 bool conv_supported(const Tensor& x, const Tensor& w, int64_t ph, int64_t pw) {
   if (!x.is_cuda() || !w.is_cuda() || x.scalar_type() != at::kFloat || w.scalar_type() != at::kFloat || x.dim() != 4 || w.dim() != 4 ||
-      !x.is_contiguous() || w.size(0) != 32 || w.size(1) != x.size(1) || x.size(0) > 65535 || !plain(x) || !plain(w))
+      !x.is_contiguous() || w.size(0) != 32 || w.size(1) != x.size(1) || x.size(0) > 65535 || !tf32_allowed() || !plain(x) || !plain(w))
     return false;
   const Conv c(x, w, ph, pw);
   return bc_conv_supported(x.device().index(), c.v) == 1;

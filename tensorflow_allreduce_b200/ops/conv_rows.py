@@ -2,7 +2,7 @@
 
 `RowConv2d` is a `torch.nn.Conv2d` (same parameters and `state_dict` keys). With 32 output channels, vertical stride 2 and
 either 32 input channels at horizontal stride 1 or one input channel at horizontal stride 2, fp32 NCHW CUDA tensors and
-TF32 convolutions allowed (`torch.backends.cudnn.allow_tf32`), it runs `csrc/cuda/conv_rows.cu` forward and backward: the tensors stay
+TF32 convolutions allowed (`torch.backends.cudnn.allow_tf32` or `.conv.fp32_precision`), it runs `csrc/cuda/conv_rows.cu` forward and backward: the tensors stay
 NCHW, TF32 operands are rounded to nearest and sums are fp32. Everything else is `F.conv2d`.
 
 The reference's pieces are Conv2D and its gradients on cuDNN (tensorflow/core/kernels/conv_ops.cc, conv_grad_filter_ops.cc,
@@ -25,7 +25,7 @@ class RowConv2d(torch.nn.Conv2d):
     """`Conv2d` whose covered forms (see the module's docstring) run on the row convolution kernels."""
 
     def _covered(self, x: torch.Tensor) -> bool:
-        if not (x.is_cuda and torch.backends.cudnn.allow_tf32 and x.dim() == 4 and x.numel() > 0) or torch.is_autocast_enabled("cuda"):
+        if not (x.is_cuda and x.dim() == 4 and x.numel() > 0) or torch.is_autocast_enabled("cuda"):
             return False
         sw = {32: 1, 1: 2}.get(self.in_channels)
         return (self.out_channels == 32 and sw is not None and self.stride == (2, sw) and self.dilation == (1, 1) and self.groups == 1

@@ -235,3 +235,16 @@ def test_dispatch_modes_see_the_operators():
     with FlopCounterMode(display=False) as stock, torch.no_grad():
         _stock(m, x, m.weight)
     assert mine.get_total_flops() == stock.get_total_flops() > 0
+
+
+def test_precision_asked_for_by_operator():
+    m, x = _conv()
+    before = torch.backends.cudnn.conv.fp32_precision
+    want = _stock(m, x.double(), m.weight.double())
+    try:
+        torch.backends.cudnn.conv.fp32_precision = "ieee"
+        _close(m(x), want, 1e-5)
+    finally:
+        torch.backends.cudnn.conv.fp32_precision = before
+    with torch.backends.cudnn.flags(enabled=False):
+        _close(m(x), want, 1e-5)
