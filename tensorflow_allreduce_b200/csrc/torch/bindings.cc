@@ -93,9 +93,17 @@ Tensor bn_clip(const Tensor& x, const Tensor& weight, const Tensor& bias, const 
                const c10::optional<Tensor>& running_var, const c10::optional<Tensor>& batches, double eps, double momentum, double clip) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 2 && x.numel() > 0,
               "bn_clip needs a contiguous fp32 CUDA tensor");
-  if (traced()) {
+  // The kernels take the channels' values, and update the counter of batches, where they lie: in memory of this device.
+  auto fits = [&](const c10::optional<Tensor>& t) {
+    return !t || (t->device() == x.device() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == x.size(1));
+  };
+  if (traced() || !fits(weight) || !fits(bias) || !fits(running_mean) || !fits(running_var)) {
     if (batches) Tensor(*batches).add_(1);
     return at::hardtanh(at::batch_norm(x, weight, bias, running_mean, running_var, true, momentum, eps, at::globalContext().userEnabledCuDNN()), 0.0, clip);
+  }
+  if (batches && (batches->device() != x.device() || batches->scalar_type() != at::kLong)) {
+    Tensor(*batches).add_(1);
+    return BnClip::apply(x, weight, bias, running_mean, running_var, c10::nullopt, eps, momentum, clip);
   }
   return BnClip::apply(x, weight, bias, running_mean, running_var, batches, eps, momentum, clip);
 }

@@ -248,3 +248,29 @@ def test_precision_asked_for_by_operator():
         torch.backends.cudnn.conv.fp32_precision = before
     with torch.backends.cudnn.flags(enabled=False):
         _close(m(x), want, 1e-5)
+
+
+def test_norm_whose_buffers_lie_elsewhere():
+    from tensorflow_allreduce_b200.ops import bn_clip
+
+    torch.manual_seed(0)
+    x = torch.randn(3, 4, 5, 6, device="cuda")
+    want = bn_clip.BatchNormClip2d(4).cuda()
+    y = want(x)
+    for count in (torch.tensor(7), torch.tensor(7, device="cuda", dtype=torch.int32), torch.tensor(7, device="cuda"), None):
+        m = bn_clip.BatchNormClip2d(4).cuda()
+        m.num_batches_tracked = count
+        before = bn_clip.launch_count
+        assert torch.equal(m(x), y) and bn_clip.launch_count == before + 1
+        assert count is None or (m.num_batches_tracked.item() == 8 and m.num_batches_tracked.device == count.device)
+        assert torch.equal(m.running_mean, want.running_mean) and torch.equal(m.running_var, want.running_var)
+    m = bn_clip.BatchNormClip2d(4).cuda()
+    both = torch.zeros(4, 2, device="cuda")
+    m.running_mean = both[:, 0]
+    m.weight = torch.nn.Parameter(torch.ones(4, 3, device="cuda")[:, 1])
+    torch.testing.assert_close(m(x), y, rtol=1e-5, atol=1e-5)
+    assert (both[:, 1] == 0).all() and m.num_batches_tracked.item() == 1
+    m = bn_clip.BatchNormClip2d(4).cuda()
+    m.running_mean = torch.zeros(4)
+    with pytest.raises(RuntimeError):
+        m(x)
