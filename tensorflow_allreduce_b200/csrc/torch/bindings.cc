@@ -125,13 +125,22 @@ int* gru_status(const Tensor& like) {
 
 // Memory through which the blocks of a launch exchange operands and partial sums. Every word says which step it belongs to
 // and a launch clears its part first, so the contents only have to be zero once. Kernels on one stream use it one after the
-// other: one buffer per device and stream.
-void* gru_scratch(const Tensor& like, void* stream, int64_t T, int64_t B, int64_t H, int64_t nd) {
+// other: one buffer per device and stream, for the 16 streams that came last. The caller holds it until its launch is queued: another
+// thread's call on the stream may want a larger one in the meantime. A captured launch has its own, cleared by the graph: two graphs may
+// run at a time, on any streams, and the second before the first.
+constexpr size_t kScratchStreams = 16;
+Tensor gru_scratch(const Tensor& like, void* stream, int64_t T, int64_t B, int64_t H, int64_t nd) {
   const int64_t need = bc_gru_scratch_bytes((int)T, (int)B, (int)H, (int)nd);
+  auto make = [&] { return at::zeros({need}, like.options().dtype(at::kByte)); };
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  C10_CUDA_CHECK(cudaStreamIsCapturing((cudaStream_t)stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) return make();
   std::lock_guard<std::mutex> g(g_gru_mu);
-  Tensor& t = g_gru_scratch[{like.device().index(), stream}];
-  if (!t.defined() || t.numel() < need) t = at::zeros({need}, like.options().dtype(at::kByte));
-  return t.data_ptr();
+  const std::pair<int, void*> key{like.device().index(), stream};
+  if (g_gru_scratch.size() >= kScratchStreams && !g_gru_scratch.count(key)) g_gru_scratch.clear();
+  Tensor& t = g_gru_scratch[key];
+  if (!t.defined() || t.numel() < need) t = make();
+  return t;
 }
 
 Tensor aligned(const Tensor& t) {
@@ -155,8 +164,9 @@ Tensor gru_run(const Tensor& x, at::TensorList w, bool save, variable_list* keep
   Tensor rsv;
   if (save) rsv = at::empty({nd, T, B, H, 4}, x.options());
   void* s = stream_of(x);
+  const Tensor scratch = gru_scratch(x, s, T, B, H, nd);
   check(bc_gru_forward((int)T, (int)B, (int)H, (int)nd, ptr(w_hh[0]), ptr(w_hh[nd - 1]), ptr(b_hh[0]), ptr(b_hh[nd - 1]), ptr(gx), ptr(y), ptr(rsv),
-                       gru_scratch(x, s, T, B, H, nd), (unsigned*)gru_status(x), g_gru_timeout_s, s),
+                       scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, s),
         "bc_gru_forward");
   g_gru_launches++;
   if (save) {
@@ -184,8 +194,9 @@ struct GruLayer : torch::autograd::Function<GruLayer> {
     // gradients of the pre-activations: (dr, dz, dn) of every direction, then dn * r of every direction
     Tensor dg = at::empty({T * B, nd * 4 * H}, x.options()), db = at::empty({nd, 2, H3}, x.options());
     void* s = stream_of(x);
+    const Tensor scratch = gru_scratch(x, s, T, B, H, nd);
     check(bc_gru_backward((int)T, (int)B, (int)H, (int)nd, ptr(saved[4]), ptr(saved[3 + nd]), ptr(y), ptr(rsv), ptr(dy), ptr(dg), ptr(db),
-                          gru_scratch(x, s, T, B, H, nd), (unsigned*)gru_status(x), g_gru_timeout_s, s),
+                          scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, s),
           "bc_gru_backward");
     g_gru_launches++;
     const Tensor dgx = dg.narrow(1, 0, nd * H3);

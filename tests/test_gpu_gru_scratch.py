@@ -1,0 +1,115 @@
+"""The memory through which the blocks of a persistent GRU layer exchange: under CUDA graphs, with several threads on a stream, with many
+streams."""
+import threading
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(H, B=5, T=12, seed=0):
+    torch.manual_seed(seed)
+    return torch.nn.GRU(24, H, bidirectional=True).cuda(), torch.randn(T, B, 24, device="cuda", requires_grad=True)
+
+
+def _pass(rnn, x):
+    from tensorflow_allreduce_b200.ops import persistent_gru as pg
+
+    y = pg.gru_forward(rnn, x)
+    return [y.detach(), *torch.autograd.grad(y, [x, *rnn.parameters()], torch.ones_like(y))]
+
+
+def test_graphs_in_any_order_and_at_a_time():
+    from tensorflow_allreduce_b200.ops import persistent_gru as pg
+
+    layers = [_layer(128, seed=1), _layer(256, seed=2)]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = [[t.clone() for t in _pass(*l)] for l in layers]
+    torch.cuda.current_stream().wait_stream(side)
+    graphs, outs = [], []
+    for l in layers:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(_pass(*l))
+        graphs.append(g)
+
+    def check(i):
+        torch.cuda.synchronize()
+        pg.check_status()
+        for a, b in zip(outs[i], want[i]):
+            assert torch.equal(a, b)
+            a.zero_()
+
+    graphs[1].replay()
+    check(1)
+    graphs[0].replay()
+    check(0)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(50):
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+    check(0)
+    check(1)
+    del graphs[0]
+    with torch.cuda.stream(side):
+        got = _pass(*layers[0])
+    torch.cuda.synchronize()
+    for a, b in zip(got, want[0]):
+        assert torch.equal(a, b)
+
+
+def test_threads_on_one_stream():
+    from tensorflow_allreduce_b200.ops import persistent_gru as pg
+
+    sizes = [(128, 2), (256, 9), (384, 17), (512, 32)]
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        layers = [_layer(h, b, 7, seed=h) for h, b in sizes]
+        want = [_pass(*l) for l in layers]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.cuda.stream(stream):
+            for _ in range(10):
+                for j in range(len(layers)):
+                    k = (i + j) % len(layers)
+                    got = _pass(*layers[k])
+                    if not all(torch.equal(a, b) for a, b in zip(got, want[k])):
+                        wrong.append(k)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    pg.check_status()
+    assert not wrong
+
+
+def test_many_streams_do_not_hold_more_and_more_memory():
+    from tensorflow_allreduce_b200 import _lib
+
+    from tensorflow_allreduce_b200.ops import persistent_gru as pg
+
+    rnn, x = _layer(1024, 32, 2)
+    size = _lib.lib().bc_gru_scratch_bytes(2, 32, 1024, 2)
+    streams = [torch.cuda.Stream() for _ in range(24)] + [torch.cuda.Stream(priority=-1) for _ in range(24)]
+    assert len({s.cuda_stream for s in streams}) > 32
+    held = []
+    with torch.no_grad():
+        for rounds in range(2):
+            for s in streams:
+                with torch.cuda.stream(s):
+                    torch.mm(x[0], x[0].t())               # torch keeps a workspace for the products of each stream
+                    if rounds:
+                        pg.gru_forward(rnn, x)
+            torch.cuda.synchronize()
+            held.append(torch.cuda.memory_allocated())
+    assert held[1] - held[0] <= 17 * size
