@@ -43,8 +43,8 @@
 //     forward): what bounds the exchange is the fresh lines, not the number of bytes in flight.
 // Microseconds per step: see choose_split().
 //
-// Every wait is bounded by %globaltimer. When a wait runs out the block records a status bit, waits
-// (bounded) for its own MMAs in flight, frees its tensor memory and returns.
+// Every wait is bounded by %globaltimer. When a wait runs out the block records a status bit, goes through its remaining steps without
+// waiting, and like every block waits (bounded) for its own MMAs in flight before it frees its tensor memory and returns.
 #include "gru_persistent.h"
 
 #include "tcgen05_prims.cuh"
@@ -186,10 +186,7 @@ __device__ __forceinline__ float tanhf_(float x) {
   return copysignf(fmaf(-m, div_(num, den), m), x);
 }
 
-// Barrier 1: all gate and loader warps have read the accumulator and sent their part of it; the loaders only arrive.
-__device__ __forceinline__ void sent_sync() { asm volatile("barrier.cta.sync 1, 512;" ::: "memory"); }
-__device__ __forceinline__ void sent_arrive() { asm volatile("barrier.cta.arrive 1, 512;" ::: "memory"); }
-__device__ __forceinline__ void gates_sync() { asm volatile("barrier.cta.sync 2, 256;" ::: "memory"); }
+__device__ __forceinline__ void gates_sync() { asm volatile("barrier.cta.sync 1, 256;" ::: "memory"); }
 
 // Where everything of one block lives; a function of the pass, the split and the dimensions.
 struct Plan {
@@ -244,7 +241,9 @@ __device__ __forceinline__ void load_weights16(const float* w, int H, int C, int
 // Three kinds of warps, so that no work off the chain of a step (output stores, prefetches) delays the next
 // product: gate warps, loader warps, and one warp that issues the MMAs. One barrier each says that
 // the operand is in shared memory (full[group]: loaders -> MMA), that the accumulator is complete (done:
-// MMA -> all), that it has been read (read: all -> MMA), and that this block has published (published: gates -> loaders).
+// MMA -> all), that it has been read and sent (read: all -> MMA and gates), and that this block has published (published: gates ->
+// loaders). No wait of the loop is a hardware barrier: those have no limit, and warps that go through the rest of their steps after a wait
+// has run out would arrive at one more often than the others.
 template <bool BWD, int C, int NB, int kLoadsPerGroup>
 __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -396,7 +395,6 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     // a few columns past the accumulator's are read as well (they are inside the allocation) and sent as padding
     tc_ld<3 * kPart>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(3 * pk_lo), v);
     tc_fence_before();
-    if (lane == 0) mbar_arrive(read_bar);
     if (row_ok) {
       if (owner == q) {
 #pragma unroll
@@ -409,6 +407,8 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
           if (i < pk_n) st_pack(o + i * kRows, make_uint4(v[3 * i], v[3 * i + 1], v[3 * i + 2], tag));
       }
     }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(read_bar);
   };
 
   if (ok && warp == kThreads / 32 - 1) {
@@ -468,11 +468,11 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
         __syncwarp();
       }
     }
-    if (!ok && leader) {
-      // A wait ran out here or in another warp. Nothing may be in flight when tensor memory is freed.
-      *abort_s = 1;
+    if (leader) {
+      if (!ok && !*abort_s) give_up(kGruTimeoutBlock);
+      // Nothing may be in flight when tensor memory is freed, whatever this or another warp has not waited for.
       tc_commit(drain_bar);
-      mbar_wait(drain_bar, 0, p.timeout_ns, nullptr);
+      mbar_drain(drain_bar, 0);
     }
     __syncwarp();
   } else if (ok && warp >= kGateThreads / 32) {
@@ -493,15 +493,14 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     const uint32_t pause = C == 1 ? read / 2 : C == 2 ? min(max(read, 300u), 600u) : C == 4 ? min(read, 300u) : max(read, (uint32_t)p.d.H / 3);
     constexpr int kSpan = kLoadsPerGroup == 4 ? 1 : 3;           // groups whose loads are in flight together
     bool good = true;
-    // Every step is gone through to the end even when a wait has run out (the waits then end at once): the gate warps count
-    // on the arrivals.
+    // Every step is gone through to the end even when a wait has run out; the waits then end at once.
     for (int s = 1; s < T; s++) {
       const uint32_t tag = (uint32_t)s, parity = (uint32_t)(s - 1) & 1;
       const uint32_t* src = src0 + (size_t)parity * ring_slot;
       // Not before this block has published its own words of the step, and then only when the others' are about to
       // arrive: polling takes L2 bandwidth from the blocks that still exchange partial sums. (Backward, H = 1024, B = 32:
       // polling all the time 6.8 us per step, from the publication on 4.75 us, with the pause 4.4 us.)
-      good = good && mbar_wait(pub_bar, parity, 4 * p.timeout_ns, abort_s);
+      if (good && !mbar_wait(pub_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutBlock);
       for (const uint32_t c0 = clock32(); clock32() - c0 < pause;) {
       }
       for (int g0 = 0; g0 < ngroups; g0 += kSpan) {
@@ -545,7 +544,6 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       if (good && !mbar_wait(done_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutMma);
       if (__all_sync(0xffffffffu, good)) send(tag, parity);
       else good = false;
-      sent_arrive();
     }
   } else if (ok) {
     // ---------------- gates ----------------
@@ -570,7 +568,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       stamp(s, 1);
       if (__all_sync(0xffffffffu, good)) send(tag, parity);
       else good = false;
-      sent_sync();
+      if (good && !mbar_wait(read_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutBlock);
       stamp(s, 2);
       if (mine > 0) {
         uint4 v[C > 1 ? C - 1 : 1][kGates];

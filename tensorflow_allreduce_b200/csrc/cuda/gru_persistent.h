@@ -31,6 +31,7 @@ struct GruDims {
 // Status bits written to status[0] by a block whose bounded wait ran out (the kernel then
 // returns early; outputs are incomplete).
 constexpr uint32_t kGruTimeoutGrid = 1u;      // waiting for the other blocks of its direction
+constexpr uint32_t kGruTimeoutBlock = 2u;     // waiting for other warps of the block
 constexpr uint32_t kGruTimeoutMma = 4u;       // waiting for the tensor core to finish
 
 // Forward. All tensors are fp32, contiguous, on the current device; w_hh, rsv and scratch 16-byte aligned.

@@ -51,6 +51,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
   }
   return true;
 }
+// Wait for what the block itself has in flight (MMAs, copies) before it frees tensor memory and ends. Microseconds, and not bounded by the
+// caller's limit: a short one would let the block end under its own work.
+__device__ __forceinline__ bool mbar_drain(uint32_t bar, uint32_t parity) { return mbar_wait(bar, parity, 1000000000ull, nullptr); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
