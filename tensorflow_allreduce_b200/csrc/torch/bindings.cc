@@ -254,21 +254,18 @@ Tensor gru_stack(Tensor x, const std::vector<Tensor>& weights, int64_t layers) {
   return x;
 }
 
-// Status of the kernels on `device` since the last call (waits for the device); 0 = fine.
+// Status of the kernels on `device` since the last call, on all of its streams (waits for the device); 0 = fine.
 int gru_take_status(int device) {
-  Tensor t;
-  {
-    std::lock_guard<std::mutex> g(g_gru_mu);
-    auto it = g_gru_status.find(device);
-    if (it == g_gru_status.end()) return 0;
-    t = it->second;
-  }
-  const int code = t.item<int>();
-  if (code) {
-    t.zero_();
-    std::lock_guard<std::mutex> g(g_gru_mu);
-    for (auto& kv : g_gru_scratch)
-      if (kv.first.first == device) kv.second.zero_();
+  std::lock_guard<std::mutex> g(g_gru_mu);
+  auto it = g_gru_status.find(device);
+  if (it == g_gru_status.end()) return 0;
+  const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  c10::cuda::device_synchronize();
+  const int code = it->second.item<int>();
+  if (code) {                     // what a launch that gave up has left in the exchange memory is not used again
+    it->second.zero_();
+    for (auto s = g_gru_scratch.begin(); s != g_gru_scratch.end();) s = s->first.first == device ? g_gru_scratch.erase(s) : std::next(s);
+    c10::cuda::device_synchronize();
   }
   return code;
 }

@@ -113,3 +113,17 @@ def test_many_streams_do_not_hold_more_and_more_memory():
             torch.cuda.synchronize()
             held.append(torch.cuda.memory_allocated())
     assert held[1] - held[0] <= 17 * size
+
+
+def test_status_is_that_of_all_streams():
+    from tensorflow_allreduce_b200.ops import persistent_gru as pg
+
+    rnn, x = _layer(128)
+    _pass(rnn, x)
+    side, done = torch.cuda.Stream(), torch.cuda.Event()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)                # about a tenth of a second
+        _pass(rnn, x)
+        done.record()
+    pg.check_status()
+    assert done.query()
