@@ -18,7 +18,7 @@
 // of rows in shared memory as the input row advances. Every block adds up a share of images and column chunks of 32 and
 // writes its partial sums; a second kernel adds the blocks' partial sums in fixed order.
 //
-// Every wait is bounded and ends in the status word.
+// Every wait is bounded and ends in the status word; a block that gives up waits for its own copies and MMAs before it ends.
 #include "conv_rows.h"
 
 #include <algorithm>
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
     }
     if (leader) tc_commit(done);      // also the end of whatever is in flight when a wait has run out
     __syncwarp();
-    ok = mbar_wait(done, 0, p.timeout_ns, nullptr) && ok;
+    ok = mbar_drain(done, 0) && ok;
   } else {
     // ---------------- weights ----------------
     if (elect_one()) {
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const __grid_cons
         }
       // No copy may be in flight when the block ends: the MMA warp has waited for all of them unless it gave up.
       for (int back = min(b, kBStages); back > 0; back--)
-        mbar_wait(b_full + 8 * ((b - back) % kBStages), (uint32_t)((b - back) / kBStages) & 1, p.timeout_ns, nullptr);
+        mbar_drain(b_full + 8 * ((b - back) % kBStages), (uint32_t)((b - back) / kBStages) & 1);
     }
     __syncwarp();
   }
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad_kernel(const __grid_co
     }
     if (leader) tc_commit(done);
     __syncwarp();
-    ok = mbar_wait(done, 0, p.timeout_ns, nullptr) && ok;
+    ok = mbar_drain(done, 0) && ok;
   }
   if (!ok) {
     *abort_s = 1;

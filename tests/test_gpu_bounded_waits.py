@@ -1,6 +1,7 @@
-"""Bounded waits of the persistent GRU kernels that run out: the meeting of a direction's blocks is given a counter that never fills, or the
+"""Bounded waits of the persistent GRU kernels and the row convolutions that run out. GRU: the meeting of a direction's blocks is given a counter that never fills, or the
 words that the blocks exchange are wiped while they are on their way. The kernels end by themselves and say so in the status word; the next
-call is right. The limit is two milliseconds."""
+call is right. The limit is two milliseconds. Convolutions: inputs that lie in pinned host memory, which take longer to load than the limit of a
+microsecond allows the tensor cores to wait for them."""
 import ctypes as C
 
 import pytest
@@ -88,3 +89,46 @@ def test_words_that_do_not_arrive(H, B, backward):
     assert any(codes)
     code, got = l.run(backward)
     assert code == 0 and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("cin", [1, 32])
+@pytest.mark.parametrize("which", ["forward", "input", "weight"])
+def test_convolution_whose_input_comes_late(which, cin):
+    from tensorflow_allreduce_b200 import _lib
+
+    if which == "input" and cin == 1:
+        pytest.skip("the gradient of a single input channel is torch's")
+    lib = _lib.lib()
+    n, h, w, k = 16, 81, 350, (21, 11)
+    sw = 1 if cin == 32 else 2
+    ho, wo = (h + 20 - 21) // 2 + 1, (w + 10 - 11) // sw + 1
+    dims = (C.c_int * 9)(n, cin, h, w, *k, 10, 5, sw)
+    torch.manual_seed(0)
+    x, dy = torch.randn(n, cin, h, w, device="cuda"), torch.randn(n, 32, ho, wo, device="cuda")
+    weight = torch.randn(32, cin, *k, device="cuda")
+    scratch = torch.empty(lib.bc_conv_scratch_bytes(dims), dtype=torch.uint8, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def run(x, dy, limit):
+        out = torch.zeros_like({"forward": dy, "input": x, "weight": weight}[which], device="cuda")
+        if which == "forward":
+            rc = lib.bc_conv_forward(dims, p(x), p(weight), p(out), p(scratch), p(status), C.c_double(limit), stream)
+        elif which == "input":
+            rc = lib.bc_conv_backward_input(dims, p(dy), p(weight), p(out), p(scratch), p(status), C.c_double(limit), stream)
+        else:
+            rc = lib.bc_conv_backward_weight(dims, p(x), p(dy), p(out), p(scratch), p(status), C.c_double(limit), stream)
+        _lib.check(rc, which)
+        code = status.item()
+        status.zero_()
+        return code, out
+
+    code, want = run(x, dy, 10.0)
+    assert code == 0
+    late = x.cpu().pin_memory(), dy.cpu().pin_memory()
+    code, got = run(*late, 10.0)                       # late, but in time
+    assert code == 0 and torch.equal(got, want)
+    assert run(*late, 1e-6)[0] == 8
+    code, got = run(x, dy, 10.0)
+    assert code == 0 and torch.equal(got, want)
