@@ -32,7 +32,7 @@ class DS2Config:
     label_len: int = 100
     persistent_rnn: bool = True  # run the GRU stack on the library's persistent tcgen05 kernels when they support the shape
     fused_norm: bool = True      # batch norm + clipped ReLU as one module on the library's two-pass kernels (ops/bn_clip.py)
-    row_conv: bool = True        # convolutions on the library's tcgen05 kernels where they cover them (ops/conv_rows.py)
+    row_conv: bool = True        # convolutions (32 channels only, ops/conv_rows.py) and the turn of their activations on the library's kernels
 
 
 class DeepSpeech2(nn.Module):
@@ -80,7 +80,7 @@ class DeepSpeech2(nn.Module):
         [frames', batch, classes]."""
         x = self.conv(spect.unsqueeze(1))                 # [B, C, F', T']
         b, c, f, t = x.shape
-        if x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and 0 < x.numel() and b <= 65535:
+        if self.cfg.row_conv and x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and 0 < x.numel() and b <= 65535:
             from .. import _lib
 
             x = _lib.ext().time_major(x)                  # [T', B, C*F']
