@@ -40,8 +40,9 @@
 //     `threadIdx.x == n` branch the same M = 64, N = 32 instruction took 55 cycles instead of 26. With two warps per
 //     scheduler every instruction of a serial chain costs four to six cycles, so the loops are kept short.
 //   * Two chains of half the batch each, meant to hide one's waits behind the other's work, were slower (4.7 us per step
-//     forward): what bounds the exchange is the fresh lines, not the number of bytes in flight.
-// Microseconds per step: see choose_split().
+//     forward where one chain took 3.8): what bounds the exchange is the fresh lines, not the number of bytes in flight.
+// Microseconds per step: see choose_split(). The variants that the comments of this file compare were measured with the code as it
+// stands, other figures of a variant that is not here any more beside the time that the kernel took then.
 //
 // Every wait is bounded by %globaltimer. When a wait runs out the block records a status bit, goes through its remaining steps without
 // waiting, and like every block waits (bounded) for its own MMAs in flight before it frees its tensor memory and returns.
@@ -235,8 +236,9 @@ __device__ __forceinline__ void load_weights16(const float* w, int H, int C, int
 }
 
 // BWD: pass; C: blocks per group; NB: N of the MMA (16 or 32, at least the batch); kLoadsPerGroup: loads of a loader thread per
-// pipeline group. With five loads or more, groups of four, one in flight, win (H = 1024, B = 32: forward 3.81 -> 3.72, backward 4.39 ->
-// 4.24 us per step: fewer polls of words that are not there yet); with fewer, pairs do (forward H = 512: 2.87 against 2.97).
+// pipeline group. With five loads or more, groups of four, one in flight, win (us per step, B = 32: H = 1024 forward 3.78 -> 3.67, backward
+// 4.48 -> 4.27, H = 512 backward 3.96 -> 3.43: fewer polls of words that are not there yet; H = 768 forward loses, 3.20 -> 3.30); with fewer,
+// pairs did (forward H = 512: 2.87 against 2.97, where pairs take 2.71 now).
 //
 // Three kinds of warps, so that no work off the chain of a step (output stores, prefetches) delays the next
 // product: gate warps, loader warps, and one warp that issues the MMAs. One barrier each says that
@@ -486,9 +488,10 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     const int mine = b < B && kt0 < tiles_mine ? (tiles_mine - kt0 + kTilesPerLoad - 1) / kTilesPerLoad : 0;
     // Cycles from a block's own publication to its first poll: about what the operand words of a step take to arrive, but
     // not so little that polls meet the partial sums of groups that are still exchanging them, and not so much that this block is the
-    // last one. Measured at 15 shapes for 55 to 160 bytes per cycle; nothing to exchange: C = 1. Against `read` alone, us per
-    // step: forward H = 1024 B = 32 3.86 -> 3.78, B = 8 2.92 -> 2.79, B = 1 2.93 -> 2.59; H = 256 B = 32 2.30 -> 2.20; both passes
-    // H = 1024 B = 1 5.95 -> 5.34; none of the 15 slower by more than 0.7 %.
+    // last one. 80 bytes per cycle out of 55 to 160 tried; nothing to exchange: C = 1. No pause / `read` alone / this rule, us per step: forward
+    // H = 1024 B = 32 3.99 / 3.70 / 3.67, B = 8 2.97 / 2.75 / 2.65, B = 1 2.91 / 2.70 / 2.58, H = 256 B = 32 2.30 / 2.22 / 2.14;
+    // backward H = 1024 B = 1 2.95 / 2.87 / 2.63. Of 36 passes (H = 128 to 1024, B = 1, 8, 32) none is slower than with `read` alone by
+    // more than 1.3 %; those of H = 128 would be 2 to 5 % faster without a pause.
     const uint32_t read = (uint32_t)(pl.ntile * B * 128) / 80;
     const uint32_t pause = C == 1 ? read / 2 : C == 2 ? min(max(read, 300u), 600u) : C == 4 ? min(read, 300u) : max(read, (uint32_t)p.d.H / 3);
     constexpr int kSpan = kLoadsPerGroup == 4 ? 1 : 3;           // groups whose loads are in flight together
@@ -499,7 +502,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       const uint32_t* src = src0 + (size_t)parity * ring_slot;
       // Not before this block has published its own words of the step, and then only when the others' are about to
       // arrive: polling takes L2 bandwidth from the blocks that still exchange partial sums. (Backward, H = 1024, B = 32:
-      // polling all the time 6.8 us per step, from the publication on 4.75 us, with the pause 4.4 us.)
+      // from the publication on 4.51 us per step, with the pause 4.27; polling all the time took 6.8 where these took 4.75 and 4.4.)
       if (good && !mbar_wait(pub_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutBlock);
       for (const uint32_t c0 = clock32(); clock32() - c0 < pause;) {
       }
@@ -787,16 +790,18 @@ bool dims_ok(const GruDims& d) {
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 // Blocks per group. Fewer blocks: more operand words to poll per block and longer MMA chains; more blocks: more partial
-// sums, and with one block per group no exchange at all. Microseconds per step (B200, both directions; B = 32 | B = 8):
+// sums, and with one block per group no exchange at all. Microseconds per step (B200, both directions; B = 32 | B = 8; "-": the weights do
+// not fit):
 //   forward   H   128          256          384          512          768          1024
-//     C = 1       1.83 | 1.56  2.28 | 1.77  2.79 | 2.07  3.43 | 2.26  4.49 | 2.91   -   | 3.57
-//     C = 2       2.09 | 1.79  2.29 | 1.84  2.64 | 2.27  2.97 | 2.35  3.37 | 2.62  4.06 | 2.93
-//     C = 4       3.39 | 2.90  3.56 | 3.04  3.62 | 2.96  3.97 | 3.12  4.29 | 3.15  4.58 | 3.44
+//     C = 1       1.72 | 1.51  2.14 | 1.73  2.64 | 1.96  2.98 | 2.25  3.90 | 3.18   -   | 3.44
+//     C = 2       2.08 | 1.83  2.31 | 1.92  2.53 | 2.01  2.71 | 2.13  3.30 | 2.42  3.67 | 2.65
 //   backward
-//     C = 2       2.66 | 2.07  3.78 | 2.41  4.35 | 3.32  5.07 | 4.00   -   |  -     -   |  -
-//     C = 4       2.51 | 2.03  2.89 | 2.45  3.24 | 2.65  3.65 | 2.85  4.39 | 3.59  5.24 | 4.17
-//     C = 8       2.67 | 2.16  3.00 | 2.42  3.55 | 2.54  3.75 | 2.66  4.09 | 2.86  4.54 | 3.10
-//     C = 16       -   |  -    4.35 | 3.48   -   |  -    5.28 | 3.60  5.49 | 3.92  5.56 | 4.04
+//     C = 2       2.51 | 2.01  3.11 | 2.39  3.81 | 3.49  4.36 | 3.74   -   |  -     -   |  -
+//     C = 4       2.45 | 2.09  2.93 | 2.39  3.21 | 2.63  3.43 | 2.83  3.95 | 3.64  4.66 | 4.00
+//     C = 8       3.47 | 2.10  3.66 | 2.35  3.77 | 2.69  3.79 | 2.95  4.07 | 3.11  4.27 | 3.19
+// The rule misses the best by 0.12 us at most (forward H = 512 B = 8, backward H = 512 B = 8 and H = 768 B = 32); at B = 1 eight blocks are
+// better than four in the backward pass from H = 384 on (2.40 against 2.48, H = 512 2.51 against 2.77). Wider groups, 4 forward and 16
+// backward, need more rows than one MMA has; they were 0.5 to 1.5 us slower.
 // (Both passes took 7.7 us per step at T = 75, B = 3, H = 512 and 9.3 at B = 32, H = 1024 when blocks exchanged through
 // counters and TMA and all weights lay in shared memory.)
 int choose_split(const GruDims& d, bool bwd) {
