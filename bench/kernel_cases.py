@@ -7,6 +7,7 @@
     python bench/kernel_cases.py --case emu_allgatherv
     python bench/kernel_cases.py --case gru [--T 350]    (one bidirectional GRU layer 2048 -> 1024, batch 32: persistent kernels vs cuDNN)
     python bench/kernel_cases.py --case bn_clip          (batch norm + clipped ReLU on [32, 32, 81, 350], the speech model's first block: fused kernels vs torch)
+    python bench/kernel_cases.py --case conv_rows        (the speech model's convolutions at batch 32: row convolution kernels vs cuDNN)
 
 Each case prints one JSON line with the CUDA-event time per launch, the algorithmic bytes moved and
 the resulting GB/s next to the measured copy bandwidth (`MEASURED_PEAKS.json` when present).
@@ -48,7 +49,7 @@ def timed(fn, iters):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--case", required=True, choices=["fused_sgd", "fused_adamw_bf16", "emu_allreduce", "emu_one_shot", "emu_allgatherv", "gru", "bn_clip"])
+    ap.add_argument("--case", required=True, choices=["fused_sgd", "fused_adamw_bf16", "emu_allreduce", "emu_one_shot", "emu_allgatherv", "gru", "bn_clip", "conv_rows"])
     ap.add_argument("--mb", type=int, default=256, help="gradient / message size in MiB")
     ap.add_argument("--iters", type=int, default=10)
     ap.add_argument("--blocks", type=int, default=0)
@@ -92,6 +93,32 @@ def main():
         out["hbm_peak_gbs"] = hbm
         out["fwd_frac_of_hbm_copy_" + src] = out["fused_fwd_gbs"] / hbm
         out["bwd_frac_of_hbm_copy_" + src] = out["fused_bwd_gbs"] / hbm
+        print(json.dumps(out))
+        return
+    if a.case == "conv_rows":
+        from tensorflow_allreduce_b200.ops import conv_rows, persistent_gru
+
+        torch.backends.cudnn.allow_tf32 = True
+        torch.manual_seed(0)
+        n = 32
+        for name, cin, h, w, k, stride, pad in (("conv1", 1, 161, 700, (41, 11), (2, 2), (20, 5)), ("conv2", 32, 81, 350, (21, 11), (2, 1), (10, 5))):
+            rows = conv_rows.RowConv2d(cin, 32, k, stride=stride, padding=pad, bias=False).cuda()
+            stock = torch.nn.Conv2d(cin, 32, k, stride=stride, padding=pad, bias=False).cuda()
+            x = torch.randn(n, cin, h, w, device="cuda", requires_grad=cin > 1)
+            dy = torch.randn_like(rows(x))
+            flop = 2 * dy.numel() * cin * k[0] * k[1]
+            for impl, m in (("rows", rows), ("cudnn", stock)):
+                y = m(x)
+                passes = {"forward": lambda: m(x.detach()), "weight": lambda: torch.autograd.grad(y, m.weight, dy, retain_graph=True)}
+                if cin > 1:
+                    passes["input"] = lambda: torch.autograd.grad(y, x, dy, retain_graph=True)
+                with torch.enable_grad():
+                    for which, fn in passes.items():
+                        ms = timed(fn, a.iters)
+                        out[f"{name}_{impl}_{which}_ms"] = round(ms, 4)
+                        if impl == "rows":
+                            out[f"{name}_{impl}_{which}_tflops"] = round(flop / ms / 1e9, 1)
+        persistent_gru.check_status()
         print(json.dumps(out))
         return
     if a.case == "gru":
