@@ -2,8 +2,9 @@
 
 `RowConv2d` is a `torch.nn.Conv2d` (same parameters and `state_dict` keys). With 32 output channels, vertical stride 2 and
 either 32 input channels at horizontal stride 1 or one input channel at horizontal stride 2, fp32 NCHW CUDA tensors and
-TF32 convolutions allowed (`torch.backends.cudnn.allow_tf32` or `.conv.fp32_precision`), it runs `csrc/cuda/conv_rows.cu` forward and backward: the tensors stay
-NCHW, TF32 operands are rounded to nearest and sums are fp32. Everything else is `F.conv2d`.
+TF32 convolutions allowed (`torch.backends.cudnn.allow_tf32` or `.conv.fp32_precision`), it runs
+`csrc/cuda/conv_rows.cu` forward and backward: the tensors stay
+NCHW, TF32 operands are rounded to nearest and sums are fp32. Everything else, other numbers of channels among it, is `F.conv2d`, on the speech model's shapes two to twenty times slower.
 
 The reference's pieces are Conv2D and its gradients on cuDNN (tensorflow/core/kernels/conv_ops.cc, conv_grad_filter_ops.cc,
 conv_grad_input_ops.cc).
