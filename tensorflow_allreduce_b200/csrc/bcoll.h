@@ -159,7 +159,7 @@ int bc_max_emulated_blocks(int device, int nranks);
  * initialised group. All tensors fp32 on the current device; the second pointer of a pair (direction 1) is
  * unused when ndir == 1; `scratch` = bc_gru_scratch_bytes() bytes, zeroed when allocated and used by one call
  * at a time; `status` = 1 uint32 that receives a non-zero code if a bounded wait ran out. `stream` is a
- * cudaStream_t. bc_gru_workspace_bytes: the partial sums that one time step exchanges. */
+ * cudaStream_t. bc_gru_workspace_bytes: an upper bound of the partial sums that one time step exchanges. */
 long long bc_gru_workspace_bytes(int T, int B, int H, int ndir);
 long long bc_gru_scratch_bytes(int T, int B, int H, int ndir);
 int bc_gru_supported(int device, int T, int B, int H, int ndir);

@@ -810,8 +810,8 @@ int choose_split(const GruDims& d, bool bwd) {
   return d.H <= (small ? 512 : 256) ? 1 : 2;
 }
 
-// Bytes of partial sums (fp32, 32 batch rows, a block's own included) that a step exchanges with the
-// widest groups that the dimensions allow: 4 blocks forward, 16 backward.
+// Bytes of partial sums (fp32, 32 batch rows, a block's own included) of a step with groups of 4 blocks forward and 16 backward, wider
+// than any that is launched.
 size_t exchange_bytes(const GruDims& d) {
   const size_t blocks = (size_t)d.ndir * (d.H / kUnits);
   const int widest = d.H / kUnits % 16 == 0 ? 16 : 8;
@@ -880,9 +880,13 @@ bool gru_persistent_supported(const GruDims& d, int device) {
 
 size_t gru_persistent_workspace_bytes(const GruDims& d) { return dims_ok(d) ? exchange_bytes(d) : 0; }
 
-// Both slots of the exchange area hold three partial sums per 16 bytes, rounded up to whole 16-byte words per row: 11 for
-// 32 batch entries, less than 3/2 of the plain size.
-size_t gru_persistent_scratch_bytes(const GruDims& d) { return dims_ok(d) ? kSyncBytes + ring_bytes(d) + 3 * exchange_bytes(d) : 0; }
+// Behind the ring every block has two slots of partial sums, three per 16 bytes, from every member of its group in the wider of the two
+// passes (its own stay in shared memory; their place is not used).
+size_t gru_persistent_scratch_bytes(const GruDims& d) {
+  if (!dims_ok(d)) return 0;
+  const size_t rows = std::max(choose_split(d, false) * RowsPerOwner<false>::value, choose_split(d, true) * RowsPerOwner<true>::value);
+  return kSyncBytes + ring_bytes(d) + (size_t)d.ndir * (d.H / kUnits) * 2 * packs_of(d.B) * rows * 16;
+}
 
 cudaError_t gru_persistent_forward(const GruDims& d, const float* const* w_hh, const float* const* b_hh, const float* gx, float* y,
                                    float* rsv, void* scratch, uint32_t* status, double timeout_s, cudaStream_t stream) {

@@ -59,8 +59,8 @@ cudaError_t gru_persistent_forward(const GruDims& d, const float* const* w_hh, c
 cudaError_t gru_persistent_backward(const GruDims& d, const float* const* w_hh, const float* y, const float* rsv, const float* dy,
                                     float* dg, float* db, void* scratch, uint32_t* status, double timeout_s, cudaStream_t stream);
 
-// Bytes of partial sums that one step exchanges (plain fp32, the widest groups), and of scratch memory that
-// a forward or backward call needs for these dimensions.
+// An upper bound of the bytes of partial sums (plain fp32) that one step exchanges, and the bytes of scratch memory that a forward or
+// backward call needs for these dimensions.
 size_t gru_persistent_workspace_bytes(const GruDims& d);
 size_t gru_persistent_scratch_bytes(const GruDims& d);
 

@@ -1,4 +1,5 @@
-"""What `persistent_gru.check_status` makes of the status words (no GPU: the extension is a stand-in)."""
+"""The host side of the persistent GRU layers without a GPU: what `persistent_gru.check_status` makes of the status words (the extension is a
+stand-in), the size of the memory through which blocks exchange."""
 import types
 
 import pytest
@@ -24,3 +25,20 @@ def test_status_words_become_errors(monkeypatch):
     codes[0] = 8
     with pytest.raises(RuntimeError, match="row convolution timed out on cuda:0"):
         pg.check_status("cuda")
+
+
+def test_scratch_holds_what_the_kernels_address(native_lib):
+    # Restated from the kernel: [direction][owner block][member of the group][slot][pack of three][row] words of 16 bytes behind the ring of
+    # [direction][slot][member][K tile of 32][batch 16 or 32][32] words and 1 KiB of counters.
+    for nd in (1, 2):
+        for H in range(128, 1025, 128):
+            for B in range(1, 33):
+                blocks, nb, need = H // 16, 16 if B <= 16 else 32, 0
+                ring = nd * 2 * (3 * H + 256) * 32 * 4
+                for backward in (False, True):
+                    small = B <= 16
+                    C = (4 if H <= (256 if small else 512) else 8) if backward else (1 if H <= (512 if small else 256) else 2)
+                    rows, kq = (16, 3 * H // C) if backward else (48, H // C)
+                    assert nd * 2 * C * -(-kq // 32) * nb * 32 * 4 <= ring
+                    need = max(need, nd * blocks * C * 2 * -(-B // 3) * rows * 16)
+                assert native_lib.bc_gru_scratch_bytes(7, B, H, nd) == 1024 + ring + need
