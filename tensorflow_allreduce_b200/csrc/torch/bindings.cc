@@ -8,6 +8,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -116,10 +117,33 @@ std::mutex g_gru_mu;
 std::map<int, Tensor> g_gru_status;                              // per device: the kernels' status word
 std::map<std::pair<int, void*>, Tensor> g_gru_scratch;           // per device and stream
 
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &status));
+  return status != cudaStreamCaptureStatusNone;
+}
+
+// Made by the first call on the device. If that is a captured one the word is made outside the capture, for good: memory of the graph
+// would be cleared by every replay, and hold anything before the first.
 int* gru_status(const Tensor& like) {
   std::lock_guard<std::mutex> g(g_gru_mu);
   Tensor& t = g_gru_status[like.device().index()];
-  if (!t.defined()) t = at::zeros({1}, like.options().dtype(at::kInt));
+  if (!t.defined()) {
+    const auto options = like.options().dtype(at::kInt);
+    if (capturing((cudaStream_t)stream_of(like))) {
+      const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+      void* word = nullptr;
+      cudaStream_t aside = nullptr;
+      C10_CUDA_CHECK(cudaMalloc(&word, sizeof(int)));
+      C10_CUDA_CHECK(cudaStreamCreateWithFlags(&aside, cudaStreamNonBlocking));
+      C10_CUDA_CHECK(cudaMemsetAsync(word, 0, sizeof(int), aside));
+      C10_CUDA_CHECK(cudaStreamSynchronize(aside));
+      C10_CUDA_CHECK(cudaStreamDestroy(aside));
+      t = at::from_blob(word, {1}, options);
+    } else {
+      t = at::zeros({1}, options);
+    }
+  }
   return t.data_ptr<int>();
 }
 
@@ -132,9 +156,7 @@ constexpr size_t kScratchStreams = 16;
 Tensor gru_scratch(const Tensor& like, void* stream, int64_t T, int64_t B, int64_t H, int64_t nd) {
   const int64_t need = bc_gru_scratch_bytes((int)T, (int)B, (int)H, (int)nd);
   auto make = [&] { return at::zeros({need}, like.options().dtype(at::kByte)); };
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  C10_CUDA_CHECK(cudaStreamIsCapturing((cudaStream_t)stream, &capturing));
-  if (capturing != cudaStreamCaptureStatusNone) return make();
+  if (capturing((cudaStream_t)stream)) return make();
   std::lock_guard<std::mutex> g(g_gru_mu);
   const std::pair<int, void*> key{like.device().index(), stream};
   if (g_gru_scratch.size() >= kScratchStreams && !g_gru_scratch.count(key)) g_gru_scratch.clear();

@@ -127,3 +127,36 @@ def test_status_is_that_of_all_streams():
         done.record()
     pg.check_status()
     assert done.query()
+
+
+def test_status_word_of_a_first_call_that_is_captured():
+    # In a process of its own: the status word is made by the first call. Memory of the graphs' pool that held other values before must not pass
+    # for it.
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from tensorflow_allreduce_b200.ops import persistent_gru as pg
+rnn, x = torch.nn.GRU(24, 128).cuda(), torch.randn(7, 5, 24, device="cuda")
+with torch.no_grad():
+    want = rnn(x)[0]
+    torch.addmm(rnn.bias_ih_l0, x[0], rnn.weight_ih_l0.t())
+    torch.cuda.synchronize()
+    first, second = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(first):
+        junk = [torch.full((60000,), 7, dtype=torch.int32, device="cuda") for _ in range(8)]
+        del junk
+    first.replay()
+    with torch.cuda.graph(second, pool=first.pool()):
+        y = pg.gru_forward(rnn, x)
+    pg.check_status()
+    second.replay()
+    pg.check_status()
+    assert (y - want).abs().max().item() < 5e-3
+print("right")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0 and "right" in res.stdout, res.stdout + res.stderr
