@@ -451,7 +451,7 @@ struct TimeMajor : torch::autograd::Function<TimeMajor> {
 Tensor time_major(const Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous() && x.scalar_type() == at::kFloat && x.dim() >= 2 && x.numel() > 0 && x.size(0) <= 65535,
               "time_major takes contiguous fp32 CUDA activations");
-  if (!plain(x)) return x.flatten(1, -2).permute({2, 0, 1}).contiguous();
+  if (!plain(x)) return (x.dim() == 2 ? x.unsqueeze(1) : x.flatten(1, -2)).permute({2, 0, 1}).contiguous();
   return TimeMajor::apply(x);
 }
 

@@ -86,6 +86,9 @@ def test_traced_time_first_order():
     traced = torch.jit.trace(lambda x: _lib.ext().time_major(x), (torch.randn(2, 3, 5, 7, device="cuda"),), check_trace=False)
     x = torch.randn(2, 3, 5, 7, device="cuda")
     assert torch.equal(traced(x), x.reshape(2, 15, 7).permute(2, 0, 1))
+    x = torch.randn(4, 6, device="cuda")
+    (grad,) = torch.autograd.functional.jvp(_lib.ext().time_major, x, x)[1:]
+    assert torch.equal(grad, x.t()[..., None]) and torch.equal(_lib.ext().time_major(x), x.t()[..., None])
 
 
 def test_traced_loss():
