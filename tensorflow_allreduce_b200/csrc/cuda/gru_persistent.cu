@@ -187,7 +187,13 @@ __device__ __forceinline__ float tanhf_(float x) {
   return copysignf(fmaf(-m, div_(num, den), m), x);
 }
 
-__device__ __forceinline__ void gates_sync() { asm volatile("barrier.cta.sync 1, 256;" ::: "memory"); }
+// Barrier 1: all gate and loader warps have read the accumulator and sent their part of it; the loaders only arrive. It has no limit, and
+// a warp that arrived twice before the others have come once would complete it without them and leave them waiting for good. So gate and
+// loader warps come to it once per step whatever waits have run out, and the loaders never before the gate warps have passed it the last
+// time: their wait for the block's publication is the one that is never skipped or cut short.
+__device__ __forceinline__ void sent_sync() { asm volatile("barrier.cta.sync 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void sent_arrive() { asm volatile("barrier.cta.arrive 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void gates_sync() { asm volatile("barrier.cta.sync 2, 256;" ::: "memory"); }
 
 // Where everything of one block lives; a function of the pass, the split and the dimensions.
 struct Plan {
@@ -236,16 +242,14 @@ __device__ __forceinline__ void load_weights16(const float* w, int H, int C, int
 }
 
 // BWD: pass; C: blocks per group; NB: N of the MMA (16 or 32, at least the batch); kLoadsPerGroup: loads of a loader thread per
-// pipeline group. With five loads or more, groups of four, one in flight, win (us per step, B = 32: H = 1024 forward 3.78 -> 3.67, backward
-// 4.48 -> 4.27, H = 512 backward 3.96 -> 3.43: fewer polls of words that are not there yet; H = 768 forward loses, 3.20 -> 3.30); with fewer,
-// pairs did (forward H = 512: 2.87 against 2.97, where pairs take 2.71 now).
+// pipeline group. With five loads or more, groups of four, one in flight, win (us per step, B = 32: H = 1024 forward 3.80 -> 3.68, backward
+// 4.43 -> 4.24, H = 512 backward 4.07 -> 3.39: fewer polls of words that are not there yet; H = 768 forward loses, 3.23 -> 3.31); with fewer,
+// pairs do (forward H = 512, B = 32: 2.80 against 2.91, B = 8: 2.24 against 2.51).
 //
 // Three kinds of warps, so that no work off the chain of a step (output stores, prefetches) delays the next
 // product: gate warps, loader warps, and one warp that issues the MMAs. One barrier each says that
 // the operand is in shared memory (full[group]: loaders -> MMA), that the accumulator is complete (done:
-// MMA -> all), that it has been read and sent (read: all -> MMA and gates), and that this block has published (published: gates ->
-// loaders). No wait of the loop is a hardware barrier: those have no limit, and warps that go through the rest of their steps after a wait
-// has run out would arrive at one more often than the others.
+// MMA -> all), that it has been read (read: all -> MMA), and that this block has published (published: gates -> loaders).
 template <bool BWD, int C, int NB, int kLoadsPerGroup>
 __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -397,6 +401,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     // a few columns past the accumulator's are read as well (they are inside the allocation) and sent as padding
     tc_ld<3 * kPart>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(3 * pk_lo), v);
     tc_fence_before();
+    if (lane == 0) mbar_arrive(read_bar);
     if (row_ok) {
       if (owner == q) {
 #pragma unroll
@@ -409,8 +414,6 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
           if (i < pk_n) st_pack(o + i * kRows, make_uint4(v[3 * i], v[3 * i + 1], v[3 * i + 2], tag));
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(read_bar);
   };
 
   if (ok && warp == kThreads / 32 - 1) {
@@ -489,21 +492,22 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
     // Cycles from a block's own publication to its first poll: about what the operand words of a step take to arrive, but
     // not so little that polls meet the partial sums of groups that are still exchanging them, and not so much that this block is the
     // last one. 80 bytes per cycle out of 55 to 160 tried; nothing to exchange: C = 1. No pause / `read` alone / this rule, us per step: forward
-    // H = 1024 B = 32 3.99 / 3.70 / 3.67, B = 8 2.97 / 2.75 / 2.65, B = 1 2.91 / 2.70 / 2.58, H = 256 B = 32 2.30 / 2.22 / 2.14;
-    // backward H = 1024 B = 1 2.95 / 2.87 / 2.63. Of 36 passes (H = 128 to 1024, B = 1, 8, 32) none is slower than with `read` alone by
-    // more than 1.3 %; those of H = 128 would be 2 to 5 % faster without a pause.
+    // H = 1024 B = 32 3.99 / 3.74 / 3.68, B = 8 3.00 / 2.88 / 2.78, B = 1 2.97 / 2.92 / 2.59, H = 256 B = 32 2.34 / 2.27 / 2.19;
+    // backward H = 1024 B = 1 2.97 / 2.91 / 2.82. Of 36 passes (H = 128 to 1024, B = 1, 8, 32) none is slower than with `read` alone by
+    // more than 1.3 %; those of H = 128 would be up to 5 % faster without a pause.
     const uint32_t read = (uint32_t)(pl.ntile * B * 128) / 80;
     const uint32_t pause = C == 1 ? read / 2 : C == 2 ? min(max(read, 300u), 600u) : C == 4 ? min(read, 300u) : max(read, (uint32_t)p.d.H / 3);
     constexpr int kSpan = kLoadsPerGroup == 4 ? 1 : 3;           // groups whose loads are in flight together
     bool good = true;
-    // Every step is gone through to the end even when a wait has run out; the waits then end at once.
+    // Every step is gone through to the end even when a wait has run out; the waits then end at once, but for the first.
     for (int s = 1; s < T; s++) {
       const uint32_t tag = (uint32_t)s, parity = (uint32_t)(s - 1) & 1;
       const uint32_t* src = src0 + (size_t)parity * ring_slot;
       // Not before this block has published its own words of the step, and then only when the others' are about to
       // arrive: polling takes L2 bandwidth from the blocks that still exchange partial sums. (Backward, H = 1024, B = 32:
-      // from the publication on 4.51 us per step, with the pause 4.27; polling all the time took 6.8 where these took 4.75 and 4.4.)
-      if (good && !mbar_wait(pub_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutBlock);
+      // from the publication on 4.45 us per step, with the pause 4.24; polling all the time took 6.8 where these took 4.75 and 4.4.)
+      // The gate warps always get there: of their waits before it each runs out once, five limits in all.
+      if (!mbar_wait(pub_bar, parity, 16 * p.timeout_ns + 1000000000ull, nullptr)) good = give_up(kGruTimeoutBlock);
       for (const uint32_t c0 = clock32(); clock32() - c0 < pause;) {
       }
       for (int g0 = 0; g0 < ngroups; g0 += kSpan) {
@@ -547,6 +551,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       if (good && !mbar_wait(done_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutMma);
       if (__all_sync(0xffffffffu, good)) send(tag, parity);
       else good = false;
+      sent_arrive();
     }
   } else if (ok) {
     // ---------------- gates ----------------
@@ -571,7 +576,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       stamp(s, 1);
       if (__all_sync(0xffffffffu, good)) send(tag, parity);
       else good = false;
-      if (good && !mbar_wait(read_bar, parity, 4 * p.timeout_ns, abort_s)) good = *abort_s ? false : give_up(kGruTimeoutBlock);
+      sent_sync();
       stamp(s, 2);
       if (mine > 0) {
         uint4 v[C > 1 ? C - 1 : 1][kGates];
@@ -793,15 +798,14 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 // sums, and with one block per group no exchange at all. Microseconds per step (B200, both directions; B = 32 | B = 8; "-": the weights do
 // not fit):
 //   forward   H   128          256          384          512          768          1024
-//     C = 1       1.72 | 1.51  2.14 | 1.73  2.64 | 1.96  2.98 | 2.25  3.90 | 3.18   -   | 3.44
-//     C = 2       2.08 | 1.83  2.31 | 1.92  2.53 | 2.01  2.71 | 2.13  3.30 | 2.42  3.67 | 2.65
+//     C = 1       1.73 | 1.43  2.19 | 1.71  2.67 | 2.00  2.88 | 2.24  3.84 | 3.12   -   | 3.51
+//     C = 2       2.05 | 1.77  2.29 | 1.92  2.64 | 2.07  2.80 | 2.23  3.32 | 2.50  3.68 | 2.78
 //   backward
-//     C = 2       2.51 | 2.01  3.11 | 2.39  3.81 | 3.49  4.36 | 3.74   -   |  -     -   |  -
-//     C = 4       2.45 | 2.09  2.93 | 2.39  3.21 | 2.63  3.43 | 2.83  3.95 | 3.64  4.66 | 4.00
-//     C = 8       3.47 | 2.10  3.66 | 2.35  3.77 | 2.69  3.79 | 2.95  4.07 | 3.11  4.27 | 3.19
-// The rule misses the best by 0.12 us at most (forward H = 512 B = 8, backward H = 512 B = 8 and H = 768 B = 32); at B = 1 eight blocks are
-// better than four in the backward pass from H = 384 on (2.40 against 2.48, H = 512 2.51 against 2.77). Wider groups, 4 forward and 16
-// backward, need more rows than one MMA has; they were 0.5 to 1.5 us slower.
+//     C = 2       2.68 | 2.00  3.14 | 2.39  3.84 | 3.53  4.55 | 3.75   -   |  -     -   |  -
+//     C = 4       2.31 | 1.88  2.90 | 2.39  3.09 | 2.59  3.40 | 2.81  3.93 | 3.61  4.59 | 4.00
+//     C = 8       3.32 | 2.16  3.47 | 2.34  3.64 | 2.63  3.69 | 2.83  4.03 | 3.05  4.24 | 3.21
+// The rule misses the best by 0.1 us at most (backward H = 768 B = 32; at B = 1 forward H = 512, 2.17 against 2.07). Wider groups, 4 forward
+// and 16 backward, need more rows than one MMA has; they were 0.5 to 1.5 us slower.
 // (Both passes took 7.7 us per step at T = 75, B = 3, H = 512 and 9.3 at B = 32, H = 1024 when blocks exchanged through
 // counters and TMA and all weights lay in shared memory.)
 int choose_split(const GruDims& d, bool bwd) {
