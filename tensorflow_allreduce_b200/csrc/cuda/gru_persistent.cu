@@ -154,13 +154,13 @@ __device__ __forceinline__ bool stale(const Words& v, uint32_t tag) {
 }
 
 // The gate functions are on the critical path of every step and bound by instruction issue: with `tanhf` and IEEE divisions, whose
-// rare cases branch, a forward step of H = 1024, B = 32 took 4.34 us, with these 3.70 (with approximate divisions alone 3.68, but tanh
+// rare cases branch, a forward step of H = 1024, B = 32 took 4.34 us, with these 3.69 (with approximate divisions alone 3.68, but tanh
 // was then off by up to 4.0 units in the last place for x < 0). Neither may be further off than CUDA's, in no range. Scan of all floats
 // against fp64, largest / mean error: tanh up to 0.62 0.84 / 0.25 units (`tanhf` 1.81 / 0.63), 0.62 to 1 1.81 / 0.38 (the same), 1 to 2
 // 1.37 / 0.28 (the same); sigmoid as 1 / (1 + __expf(-x)) everywhere: 1.6 for x > 0, 8.4 at -8, 62 at -80, the rounding of x log2 e.
-__device__ __forceinline__ float div_(float a, float b) {
+__device__ __forceinline__ float rcp_(float x) {
   float y;
-  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 __device__ __forceinline__ float exp2_(float x) {
@@ -169,10 +169,10 @@ __device__ __forceinline__ float exp2_(float x) {
   return y;
 }
 // 1 / (1 + e^-x) as a quarter of the reciprocal of a quarter of the denominator, so that neither leaves the normal range before the
-// result does; one step of Newton's method, y + y (1 - d y), takes the division's error out.
+// result does; one step of Newton's method, y + y (1 - d y), takes the approximation's error out.
 __device__ __forceinline__ float sigmoidf_(float x) {
   const float d = fmaf(exp2_(x * -1.44269504f), 0.25f, 0.25f);
-  const float y = div_(1.f, d);
+  const float y = rcp_(d);
   return d < INFINITY ? 0.25f * fmaf(y, fmaf(-d, y, 1.f), y) : y;
 }
 // sign(x) (1 - 2 / (1 + e^2|x|)); where that cancels, Lambert's continued fraction cut behind its fifth partial denominator as
@@ -184,7 +184,7 @@ __device__ __forceinline__ float tanhf_(float x) {
   const float num = small ? q * fmaf(q, 14.f, 315.f) : 2.f;
   const float den = small ? fmaf(q, fmaf(q, 15.f, 420.f), 945.f) : 1.f + exp2_(a * 2.88539008f);
   const float m = small ? a : 1.f;
-  return copysignf(fmaf(-m, div_(num, den), m), x);
+  return copysignf(fmaf(-m, num * rcp_(den), m), x);
 }
 
 // Barrier 1: all gate and loader warps have read the accumulator and sent their part of it; the loaders only arrive. It has no limit, and
