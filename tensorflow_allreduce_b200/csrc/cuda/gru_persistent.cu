@@ -1,4 +1,5 @@
-// Persistent bidirectional GRU layer for sm_100a (see gru_persistent.h for the interface).
+// Persistent bidirectional GRU layer for sm_100a (see gru_persistent.h for the interface): backward pass and host side. The forward
+// pass is in gru_forward.cu.
 //
 // Work split. Direction d of a layer is run by H/16 blocks (grid.y = direction); block c owns
 // the hidden units [16c, 16c+16) and produces their outputs. For the recurrent product the blocks
@@ -46,9 +47,7 @@
 //
 // Every wait is bounded by %globaltimer. When a wait runs out the block records a status bit, goes through its remaining steps without
 // waiting, and like every block waits (bounded) for its own MMAs in flight before it frees its tensor memory and returns.
-#include "gru_persistent.h"
-
-#include "tcgen05_prims.cuh"
+#include "gru_common.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -58,44 +57,17 @@ namespace gpu {
 
 namespace {
 
-using namespace tc;
+using namespace gru;
 
-constexpr int kUnits = 16;            // hidden units per block
 constexpr int kKTile = 32;            // fp32 elements in one 128-byte swizzle row
 constexpr int kGateThreads = 256;     // eight warps: accumulator read-back, exchange, gate math
 constexpr int kLoadThreads = 256;     // eight warps: poll the operand words and put them into shared memory
 constexpr int kThreads = kGateThreads + kLoadThreads + 32;   // and the warp that issues the MMAs
 constexpr int kMaxBlocksPerDir = 64;  // H / 16 at H = 1024
-constexpr uint32_t kTmemCols = 512;
 constexpr int kLoadBytes = kLoadThreads * 32;   // operand bytes that one load of every loader thread brings
 constexpr int kMaxGroups = 8;         // pipeline groups (one mbarrier each) of a step: 32 K tiles of 32 batch rows in pairs of loads
-constexpr int kMinSmem = 120 * 1024;  // more than half of an SM's shared memory: one block per SM, since a block takes all of tensor memory
-
-struct Params {
-  GruDims d;
-  const float* w_hh[2];   // [3H, H] of each direction
-  const float* b_hh[2];   // forward: [3H] of each direction
-  const float* gx;        // forward
-  float* y;               // forward: out; backward: in (const)
-  float4* rsv;            // forward: out, or null; backward: in
-  const float* dy;        // backward
-  float* dg;              // backward: out
-  float* db;              // backward: out
-  uint32_t* ring;         // operand words: [dir][slot 2][member C][K tile][batch NB][32]
-  uint4* xchg;            // partial sums: [dir][owner block][source C][slot 2][pack][row] x 16 bytes
-  uint32_t* sync;         // per direction: arrivals, generation
-  uint32_t* status;
-  unsigned long long timeout_ns;
-  unsigned long long* prof;   // optional: 8 time stamps per step of block (0, 0), for tuning
-};
-
 // ---- PTX wrappers beside those of tcgen05_prims.cuh ---------------------------------------------
 
-__device__ __forceinline__ uint32_t clock32() {
-  uint32_t c;
-  asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
-  return c;
-}
 // N consecutive columns of this thread's tensor-memory lane: the packs that one warp reads back (see `send` below).
 template <int N> __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t* r);
 template <> __device__ __forceinline__ void tc_ld<6>(uint32_t taddr, uint32_t* r) {
@@ -116,18 +88,6 @@ template <> __device__ __forceinline__ void tc_ld<9>(uint32_t taddr, uint32_t* r
 }
 // Words that travel between blocks.
 __device__ __forceinline__ void st_word(uint32_t* p, uint32_t v) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
-// 32 bytes per request: a strong load costs L2 the same whatever its width (fresh lines, 32 KB per block and 128 blocks:
-// 1406 cycles this way, 1758 with 16-byte loads).
-struct Words { uint32_t w[8]; };
-// Two neighbouring chunks of a swizzled row: the second one's place differs in bit 4.
-__device__ __forceinline__ void st_shared2(uint32_t at, const Words& v) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]), "r"(v.w[3]) : "memory");
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at ^ 16), "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]), "r"(v.w[7]) : "memory");
-}
-__device__ __forceinline__ void ld_words(const uint32_t* p, Words& v) {
-  asm volatile("ld.relaxed.gpu.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p) : "memory");
-}
 __device__ __forceinline__ void st_pack(uint4* p, uint4 v) {
   asm volatile(
       "{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
@@ -153,40 +113,6 @@ __device__ __forceinline__ bool stale(const Words& v, uint32_t tag) {
   return (d & kTagMask) != 0;
 }
 
-// The gate functions are on the critical path of every step and bound by instruction issue: with `tanhf` and IEEE divisions, whose
-// rare cases branch, a forward step of H = 1024, B = 32 took 4.34 us, with these 3.69 (with approximate divisions alone 3.68, but tanh
-// was then off by up to 4.0 units in the last place for x < 0). Neither may be further off than CUDA's, in no range. Scan of all floats
-// against fp64, largest / mean error: tanh up to 0.62 0.84 / 0.25 units (`tanhf` 1.81 / 0.63), 0.62 to 1 1.81 / 0.38 (the same), 1 to 2
-// 1.37 / 0.28 (the same); sigmoid as 1 / (1 + __expf(-x)) everywhere: 1.6 for x > 0, 8.4 at -8, 62 at -80, the rounding of x log2 e.
-__device__ __forceinline__ float rcp_(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float exp2_(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// 1 / (1 + e^-x) as a quarter of the reciprocal of a quarter of the denominator, so that neither leaves the normal range before the
-// result does; one step of Newton's method, y + y (1 - d y), takes the approximation's error out.
-__device__ __forceinline__ float sigmoidf_(float x) {
-  const float d = fmaf(exp2_(x * -1.44269504f), 0.25f, 0.25f);
-  const float y = rcp_(d);
-  return d < INFINITY ? 0.25f * fmaf(y, fmaf(-d, y, 1.f), y) : y;
-}
-// sign(x) (1 - 2 / (1 + e^2|x|)); where that cancels, Lambert's continued fraction cut behind its fifth partial denominator as
-// x - x v with v = q (315 + 14 q) / (945 + 420 q + 15 q^2), q = x^2: off by 7e-10 at 0.625, and the rounding of v, which is
-// below 0.12, hardly shows.
-__device__ __forceinline__ float tanhf_(float x) {
-  const float q = x * x, a = fabsf(x);
-  const bool small = q < 0.39f;
-  const float num = small ? q * fmaf(q, 14.f, 315.f) : 2.f;
-  const float den = small ? fmaf(q, fmaf(q, 15.f, 420.f), 945.f) : 1.f + exp2_(a * 2.88539008f);
-  const float m = small ? a : 1.f;
-  return copysignf(fmaf(-m, num * rcp_(den), m), x);
-}
-
 // Barrier 1: all gate and loader warps have read the accumulator and sent their part of it; the loaders only arrive. It has no limit, and
 // a warp that arrived twice before the others have come once would complete it without them and leave them waiting for good. So gate and
 // loader warps come to it once per step whatever waits have run out, and the loaders never before the gate warps have passed it the last
@@ -205,43 +131,32 @@ struct Plan {
   __host__ __device__ int smem() const { return 1024 + x_bytes + w_bytes + own_bytes + 256; }
 };
 __host__ __device__ constexpr int packs_of(int batch) { return (batch + 2) / 3; }   // three partial sums and the step number per 16 bytes
-template <bool BWD> struct RowsPerOwner { static constexpr int value = BWD ? kUnits : 3 * kUnits; };
 
-template <bool BWD>
 __host__ __device__ inline Plan make_plan(int C, int nb, int H) {
   Plan p;
-  const int rows = RowsPerOwner<BWD>::value * C;
-  p.kq = (BWD ? 3 * H : H) / C;
+  const int rows = kUnits * C;
+  p.kq = 3 * H / C;
   p.ntile = (p.kq + kKTile - 1) / kKTile;
   p.m = rows > 64 ? 128 : 64;
   const int room = (int)kTmemCols - nb;                 // the accumulator takes the first nb columns
   p.k_tmem = p.kq <= room ? p.kq : room / kKTile * kKTile;
   p.x_bytes = p.ntile * nb * 128;
   p.w_bytes = (p.kq - p.k_tmem + kKTile - 1) / kKTile * p.m * 128;
-  p.own_bytes = RowsPerOwner<BWD>::value * packs_of(nb) * 16;
+  p.own_bytes = kUnits * packs_of(nb) * 16;
   return p;
 }
 
 // The 16 weights of row `r` of the group at columns k0 .. k0 + 15 of member q's K range (k0 a multiple of 16).
-//   forward : rows ordered owner, gate, unit; K = hidden units            W[g * H + unit][q * kq + k]
-//   backward: rows ordered owner, unit; K ordered gate, unit of the range   W[g * H + unit'][unit]
+// Rows ordered owner, unit; K ordered gate, unit of the range   W[g * H + unit'][unit]
 // A run of 16 columns stays inside one gate, because a member's range of units is a multiple of 16.
-template <bool BWD>
-__device__ __forceinline__ void load_weights16(const float* w, int H, int C, int grp, int q, int kq, int r, int k0, float* o) {
-  if (!BWD) {
-    const int m = r / 48, g = (r % 48) / kUnits, u = r % kUnits;
-    const float4* p = reinterpret_cast<const float4*>(w + (size_t)(g * H + (grp * C + m) * kUnits + u) * H + q * kq + k0);
+__device__ __forceinline__ void load_weights16(const float* w, int H, int C, int grp, int q, int r, int k0, float* o) {
+  const int range = H / C, g = k0 / range, kk = q * range + k0 - g * range;
+  const float* p = w + (size_t)(g * H + kk) * H + grp * C * kUnits + r;
 #pragma unroll
-    for (int i = 0; i < 4; i++) reinterpret_cast<float4*>(o)[i] = __ldg(p + i);
-  } else {
-    const int range = H / C, g = k0 / range, kk = q * range + k0 - g * range;
-    const float* p = w + (size_t)(g * H + kk) * H + grp * C * kUnits + r;
-#pragma unroll
-    for (int i = 0; i < 16; i++) o[i] = __ldg(p + (size_t)i * H);
-  }
+  for (int i = 0; i < 16; i++) o[i] = __ldg(p + (size_t)i * H);
 }
 
-// BWD: pass; C: blocks per group; NB: N of the MMA (16 or 32, at least the batch); kLoadsPerGroup: loads of a loader thread per
+// C: blocks per group; NB: N of the MMA (16 or 32, at least the batch); kLoadsPerGroup: loads of a loader thread per
 // pipeline group. With five loads or more, groups of four, one in flight, win (us per step, B = 32: H = 1024 forward 3.80 -> 3.68, backward
 // 4.43 -> 4.24, H = 512 backward 4.07 -> 3.39: fewer polls of words that are not there yet; H = 768 forward loses, 3.23 -> 3.31); with fewer,
 // pairs do (forward H = 512, B = 32: 2.80 against 2.91, B = 8: 2.24 against 2.51).
@@ -250,22 +165,22 @@ __device__ __forceinline__ void load_weights16(const float* w, int H, int C, int
 // product: gate warps, loader warps, and one warp that issues the MMAs. One barrier each says that
 // the operand is in shared memory (full[group]: loaders -> MMA), that the accumulator is complete (done:
 // MMA -> all), that it has been read (read: all -> MMA), and that this block has published (published: gates -> loaders).
-template <bool BWD, int C, int NB, int kLoadsPerGroup>
-__global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __grid_constant__ Params p) {
+template <int C, int NB, int kLoadsPerGroup>
+__global__ void __launch_bounds__(kThreads, 1) gru_backward_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
 
-  constexpr int kRows = RowsPerOwner<BWD>::value;
+  constexpr int kRows = kUnits;            // accumulator rows of a member
   constexpr int R = kRows * C;
-  constexpr int kGates = BWD ? 1 : 3;      // accumulator rows per unit
-  constexpr int kGateWords = BWD ? 3 : 1;  // operand words that a (unit, batch) pair publishes per step
+  constexpr int kGates = 1;                // accumulator rows per unit
+  constexpr int kGateWords = 3;            // operand words that a (unit, batch) pair publishes per step
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dir = blockIdx.y, u0 = blockIdx.x * kUnits;
   const int T = p.d.T, B = p.d.B, H = p.d.H, ND = p.d.ndir;
   const int nblocks = gridDim.x;
   const int grp = blockIdx.x / C, q = blockIdx.x % C;
-  const Plan pl = make_plan<BWD>(C, NB, H);
+  const Plan pl = make_plan(C, NB, H);
   const int npacks = packs_of(B);
 
   uint8_t* x_s = smem;
@@ -343,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       float v[16];
 #pragma unroll
       for (int i = 0; i < 16; i++) v[i] = 0.f;
-      if (row_ok) load_weights16<BWD>(w, H, C, grp, q, pl.kq, lane_row, k0, v);
+      if (row_ok) load_weights16(w, H, C, grp, q, lane_row, k0, v);
       __syncwarp();
       tmem_st16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(NB + k0), v);
     }
@@ -353,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       float v[16];
 #pragma unroll
       for (int e = 0; e < 16; e++) v[e] = 0.f;
-      if (r < R) load_weights16<BWD>(w, H, C, grp, q, pl.kq, r, pl.k_tmem + k, v);
+      if (r < R) load_weights16(w, H, C, grp, q, r, pl.k_tmem + k, v);
       uint8_t* row = w_s + ((k >> 5) * pl.m + r) * 128;
 #pragma unroll
       for (int e = 0; e < 4; e++)
@@ -633,148 +548,92 @@ __global__ void __launch_bounds__(kThreads, 1) gru_persistent_kernel(const __gri
       if (lane == 0) mbar_arrive(pub_bar);
     };
 
-    if (!BWD) {
-      const float bias_r = p.b_hh[dir][u0 + u], bias_z = p.b_hh[dir][H + u0 + u], bias_n = p.b_hh[dir][2 * H + u0 + u];
-      // Running pointers: one step of time further per step of the loop, backwards for direction 1.
-      const ptrdiff_t step = dir ? -1 : 1;
-      const int t_first = dir ? T - 1 : 0;
-      const int gx_row = ND * 3 * H, y_row = ND * H;
-      const float* gx_p = p.gx + ((size_t)t_first * B + b0) * gx_row + dir * 3 * H + u0 + u;
-      float* y_p = p.y + ((size_t)t_first * B + b0) * y_row + dir * H + u0 + u;
-      float4* rsv_p = p.rsv ? p.rsv + ((size_t)(dir * T + t_first) * B + b0) * H + u0 + u : nullptr;
-      uint32_t* ring_p = ring + ring_at(0, u, b0);
-      float gx[3][3];
-      auto load_gx = [&]() {
+    const ptrdiff_t step = dir ? 1 : -1;
+    const int t_first = dir ? 0 : T - 1;
+    const int y_row = ND * H, dg_row = ND * 4 * H;
+    const float4* rsv_p = p.rsv + ((size_t)(dir * T + t_first) * B + b0) * H + u0 + u;
+    const float* dy_p = p.dy + ((size_t)t_first * B + b0) * y_row + dir * H + u0 + u;
+    const float* hp_p = p.y + ((ptrdiff_t)t_first + step) * B * y_row + (ptrdiff_t)b0 * y_row + dir * H + u0 + u;   // h of the step before in the forward pass
+    float* dg_p = p.dg + ((size_t)t_first * B + b0) * dg_row + dir * 3 * H + u0 + u;
+    const int dnr_off = (ND * 3 - dir * 2) * H;       // from (dir * 3) * H to (ND * 3 + dir) * H
+    uint32_t* ring_p[3] = {ring + ring_at(0, u, b0), ring + ring_at(1, u, b0), ring + ring_at(2, u, b0)};
+    float4 in_a[3];                                   // r, z, n, W_hn h + b_hn
+    float in_hp[3] = {0.f, 0.f, 0.f}, in_dy[3];
+    auto load_inputs = [&](bool has_prev) {
 #pragma unroll
-        for (int j = 0; j < 3; j++)
-          if (j < mine) {
-            const float* g = gx_p + j * gx_row;
-            gx[0][j] = __ldg(g); gx[1][j] = __ldg(g + H); gx[2][j] = __ldg(g + 2 * H);
-          }
-        gx_p += step * B * gx_row;
-      };
-      load_gx();
-      for (int s = 0; s < T; s++) {
-        float acc[3][3] = {};
-        stamp(s, 0);
-        if (s > 0) product(s - 1, s, acc);
-        float4 keep[3];
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          const float hn = bias_n + acc[2][j];
-          const float r_ = sigmoidf_(gx[0][j] + (bias_r + acc[0][j]));
-          const float z = sigmoidf_(gx[1][j] + (bias_z + acc[1][j]));
-          const float n = tanhf_(gx[2][j] + r_ * hn);
-          carry[j] = n + z * (carry[j] - n);
-          keep[j] = make_float4(r_, z, n, hn);
+      for (int j = 0; j < 3; j++)
+        if (j < mine) {
+          in_a[j] = __ldg(rsv_p + j * H);
+          in_dy[j] = __ldg(dy_p + j * y_row);
+          in_hp[j] = has_prev ? __ldg(hp_p + j * y_row) : 0.f;
         }
-        if (s + 1 < T) {
-          uint32_t* o = ring_p + ((s & 1) ? ring_slot : 0u);
+      rsv_p += step * B * H;
+      dy_p += step * B * y_row;
+      hp_p += step * B * y_row;
+    };
+    float sum[4] = {0.f, 0.f, 0.f, 0.f}, part[4] = {0.f, 0.f, 0.f, 0.f};   // bias gradients, in runs of 16 steps
+    load_inputs(T > 1);
+    for (int s = 0; s < T; s++) {
+      float keep[3], g[4][3];
+      stamp(s, 0);
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        const float r_ = in_a[j].x, z = in_a[j].y, n = in_a[j].z, hn = in_a[j].w;
+        const float dh = in_dy[j] + carry[j];
+        const float dn = dh * (1.f - z) * (1.f - n * n);
+        g[0][j] = dn * hn * r_ * (1.f - r_);
+        g[1][j] = dh * (in_hp[j] - n) * z * (1.f - z);
+        g[2][j] = dn;
+        g[3][j] = dn * r_;
+        keep[j] = dh * z;
+      }
+      if (s + 1 < T) {
+        const uint32_t slot = (s & 1) ? ring_slot : 0u;
+#pragma unroll
+        for (int k = 0; k < 3; k++)
 #pragma unroll
           for (int j = 0; j < 3; j++)
-            if (j < mine) st_word(o + j * kKTile, tagged(carry[j], (uint32_t)s + 1));
-          published();
-        }
-        stamp(s, 4);
-        // The peers do not wait for what follows.
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-          if (j < mine) {
-            y_p[j * y_row] = carry[j];
-            if (rsv_p) rsv_p[j * H] = keep[j];
-          }
-        y_p += step * B * y_row;
-        if (rsv_p) rsv_p += step * B * H;
-        if (s + 1 < T) load_gx();
+            if (j < mine) st_word(ring_p[k] + slot + j * kKTile, tagged(g[k == 2 ? 3 : k][j], (uint32_t)s + 1));
+        published();
       }
-    } else {
-      const ptrdiff_t step = dir ? 1 : -1;
-      const int t_first = dir ? 0 : T - 1;
-      const int y_row = ND * H, dg_row = ND * 4 * H;
-      const float4* rsv_p = p.rsv + ((size_t)(dir * T + t_first) * B + b0) * H + u0 + u;
-      const float* dy_p = p.dy + ((size_t)t_first * B + b0) * y_row + dir * H + u0 + u;
-      const float* hp_p = p.y + ((ptrdiff_t)t_first + step) * B * y_row + (ptrdiff_t)b0 * y_row + dir * H + u0 + u;   // h of the step before in the forward pass
-      float* dg_p = p.dg + ((size_t)t_first * B + b0) * dg_row + dir * 3 * H + u0 + u;
-      const int dnr_off = (ND * 3 - dir * 2) * H;       // from (dir * 3) * H to (ND * 3 + dir) * H
-      uint32_t* ring_p[3] = {ring + ring_at(0, u, b0), ring + ring_at(1, u, b0), ring + ring_at(2, u, b0)};
-      float4 in_a[3];                                   // r, z, n, W_hn h + b_hn
-      float in_hp[3] = {0.f, 0.f, 0.f}, in_dy[3];
-      auto load_inputs = [&](bool has_prev) {
+      stamp(s, 4);
+      // The peers do not wait for what follows.
 #pragma unroll
-        for (int j = 0; j < 3; j++)
-          if (j < mine) {
-            in_a[j] = __ldg(rsv_p + j * H);
-            in_dy[j] = __ldg(dy_p + j * y_row);
-            in_hp[j] = has_prev ? __ldg(hp_p + j * y_row) : 0.f;
-          }
-        rsv_p += step * B * H;
-        dy_p += step * B * y_row;
-        hp_p += step * B * y_row;
-      };
-      float sum[4] = {0.f, 0.f, 0.f, 0.f}, part[4] = {0.f, 0.f, 0.f, 0.f};   // bias gradients, in runs of 16 steps
-      load_inputs(T > 1);
-      for (int s = 0; s < T; s++) {
-        float keep[3], g[4][3];
-        stamp(s, 0);
+      for (int j = 0; j < 3; j++)
+        if (j < mine) {
+          float* o = dg_p + j * dg_row;
 #pragma unroll
-        for (int j = 0; j < 3; j++) {
-          const float r_ = in_a[j].x, z = in_a[j].y, n = in_a[j].z, hn = in_a[j].w;
-          const float dh = in_dy[j] + carry[j];
-          const float dn = dh * (1.f - z) * (1.f - n * n);
-          g[0][j] = dn * hn * r_ * (1.f - r_);
-          g[1][j] = dh * (in_hp[j] - n) * z * (1.f - z);
-          g[2][j] = dn;
-          g[3][j] = dn * r_;
-          keep[j] = dh * z;
+          for (int k = 0; k < 3; k++) o[k * H] = g[k][j];
+          o[dnr_off] = g[3][j];
+#pragma unroll
+          for (int k = 0; k < 4; k++) part[k] += g[k][j];
         }
-        if (s + 1 < T) {
-          const uint32_t slot = (s & 1) ? ring_slot : 0u;
+      dg_p += step * B * dg_row;
+      if ((s & 15) == 15) {
 #pragma unroll
-          for (int k = 0; k < 3; k++)
-#pragma unroll
-            for (int j = 0; j < 3; j++)
-              if (j < mine) st_word(ring_p[k] + slot + j * kKTile, tagged(g[k == 2 ? 3 : k][j], (uint32_t)s + 1));
-          published();
-        }
-        stamp(s, 4);
-        // The peers do not wait for what follows.
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-          if (j < mine) {
-            float* o = dg_p + j * dg_row;
-#pragma unroll
-            for (int k = 0; k < 3; k++) o[k * H] = g[k][j];
-            o[dnr_off] = g[3][j];
-#pragma unroll
-            for (int k = 0; k < 4; k++) part[k] += g[k][j];
-          }
-        dg_p += step * B * dg_row;
-        if ((s & 15) == 15) {
-#pragma unroll
-          for (int k = 0; k < 4; k++) { sum[k] += part[k]; part[k] = 0.f; }
-        }
-        if (s + 1 < T) {
-          load_inputs(s + 2 < T);
-          float acc[1][3] = {};
-          product(s, s, acc);
-#pragma unroll
-          for (int j = 0; j < 3; j++) carry[j] = keep[j] + acc[0][j];
-        }
+        for (int k = 0; k < 4; k++) { sum[k] += part[k]; part[k] = 0.f; }
       }
-      // Bias gradients of this block's units. The operand area is free: every MMA has been waited for.
-      float* red = reinterpret_cast<float*>(x_s);
-      if (mine > 0)
+      if (s + 1 < T) {
+        load_inputs(s + 2 < T);
+        float acc[1][3] = {};
+        product(s, s, acc);
 #pragma unroll
-        for (int k = 0; k < 4; k++) red[(pk * 4 + k) * kUnits + u] = sum[k] + part[k];
-      gates_sync();
-      if (tid < 4 * kUnits) {
-        float v = 0.f;
-        for (int i = 0; i < npacks; i++) v += red[i * 4 * kUnits + tid];
-        const int k = tid / kUnits;
-        float* o = p.db + dir * 6 * H + u0 + tid % kUnits;
-        if (k != 3) o[k * H] = v;                        // dr, dz, dn
-        if (k != 2) o[(k == 3 ? 5 : k + 3) * H] = v;     // dr, dz, dn * r
+        for (int j = 0; j < 3; j++) carry[j] = keep[j] + acc[0][j];
       }
+    }
+    // Bias gradients of this block's units. The operand area is free: every MMA has been waited for.
+    float* red = reinterpret_cast<float*>(x_s);
+    if (mine > 0)
+#pragma unroll
+      for (int k = 0; k < 4; k++) red[(pk * 4 + k) * kUnits + u] = sum[k] + part[k];
+    gates_sync();
+    if (tid < 4 * kUnits) {
+      float v = 0.f;
+      for (int i = 0; i < npacks; i++) v += red[i * 4 * kUnits + tid];
+      const int k = tid / kUnits;
+      float* o = p.db + dir * 6 * H + u0 + tid % kUnits;
+      if (k != 3) o[k * H] = v;                        // dr, dz, dn
+      if (k != 2) o[(k == 3 ? 5 : k + 3) * H] = v;     // dr, dz, dn * r
     }
   }
 
@@ -819,18 +678,18 @@ int choose_split(const GruDims& d, bool bwd) {
 size_t exchange_bytes(const GruDims& d) {
   const size_t blocks = (size_t)d.ndir * (d.H / kUnits);
   const int widest = d.H / kUnits % 16 == 0 ? 16 : 8;
-  return blocks * 32 * 4 * std::max(4 * RowsPerOwner<false>::value, widest * RowsPerOwner<true>::value);
+  return blocks * 32 * 4 * std::max(4 * 48, widest * kUnits);
 }
 constexpr size_t kSyncBytes = 1024;
 // Both slots of the ring. The backward pass is the larger one: three words per unit and batch entry, and the last K tile of
 // a member may be half empty.
 size_t ring_bytes(const GruDims& d) { return (size_t)d.ndir * 2 * (3 * d.H + 16 * 16) * 32 * 4; }
 
-template <bool BWD, int C, int NB, int LPG>
+template <int C, int NB, int LPG>
 cudaError_t launch_with(const Params& p, cudaStream_t stream) {
   const GruDims& d = p.d;
-  const Plan pl = make_plan<BWD>(C, NB, d.H);
-  auto kernel = gru_persistent_kernel<BWD, C, NB, LPG>;
+  const Plan pl = make_plan(C, NB, d.H);
+  auto kernel = gru_backward_kernel<C, NB, LPG>;
   const int smem = std::max(pl.smem(), kMinSmem);
   dim3 grid(d.H / kUnits, d.ndir), block(kThreads);
   if (grid.x > (unsigned)kMaxBlocksPerDir || grid.x % C != 0 || (pl.ntile + 64 / NB - 1) / (64 / NB) > LPG * kMaxGroups) return cudaErrorInvalidValue;
@@ -847,26 +706,25 @@ cudaError_t launch_with(const Params& p, cudaStream_t stream) {
   return cudaLaunchCooperativeKernel((const void*)kernel, grid, block, args, (size_t)smem, stream);
 }
 
-template <bool BWD, int C, int NB>
+template <int C, int NB>
 cudaError_t launch_as(const Params& p, cudaStream_t stream) {
-  const int loads = (make_plan<BWD>(C, NB, p.d.H).ntile + 64 / NB - 1) / (64 / NB);
-  if constexpr (BWD || C > 1)            // alone in its group a forward block never has more than four
-    if (loads >= 5) return launch_with<BWD, C, NB, 4>(p, stream);
-  return launch_with<BWD, C, NB, 2>(p, stream);
+  const int loads = (make_plan(C, NB, p.d.H).ntile + 64 / NB - 1) / (64 / NB);
+  return loads >= 5 ? launch_with<C, NB, 4>(p, stream) : launch_with<C, NB, 2>(p, stream);
 }
 
-template <bool BWD>
-cudaError_t launch(Params& p, void* scratch, double timeout_s, cudaStream_t stream) {
+void fill(Params& p, void* scratch, double timeout_s) {
   char* w = (char*)scratch;
   p.sync = (uint32_t*)w;
   p.ring = (uint32_t*)(w + kSyncBytes);
   p.xchg = (uint4*)(w + kSyncBytes + ring_bytes(p.d));
   p.timeout_ns = (unsigned long long)(timeout_s * 1e9);
   p.prof = g_prof;
-  const bool wide = choose_split(p.d, BWD) > (BWD ? 4 : 1);
-  constexpr int lo = BWD ? 4 : 1, hi = BWD ? 8 : 2;
-  if (p.d.B <= 16) return wide ? launch_as<BWD, hi, 16>(p, stream) : launch_as<BWD, lo, 16>(p, stream);
-  return wide ? launch_as<BWD, hi, 32>(p, stream) : launch_as<BWD, lo, 32>(p, stream);
+}
+
+cudaError_t launch_backward(const Params& p, cudaStream_t stream) {
+  const bool wide = choose_split(p.d, true) > 4;
+  if (p.d.B <= 16) return wide ? launch_as<8, 16>(p, stream) : launch_as<4, 16>(p, stream);
+  return wide ? launch_as<8, 32>(p, stream) : launch_as<4, 32>(p, stream);
 }
 
 }  // namespace
@@ -888,7 +746,7 @@ size_t gru_persistent_workspace_bytes(const GruDims& d) { return dims_ok(d) ? ex
 // passes (its own stay in shared memory; their place is not used).
 size_t gru_persistent_scratch_bytes(const GruDims& d) {
   if (!dims_ok(d)) return 0;
-  const size_t rows = std::max(choose_split(d, false) * RowsPerOwner<false>::value, choose_split(d, true) * RowsPerOwner<true>::value);
+  const size_t rows = std::max(choose_split(d, false) * 48, choose_split(d, true) * kUnits);
   return kSyncBytes + ring_bytes(d) + (size_t)d.ndir * (d.H / kUnits) * 2 * packs_of(d.B) * rows * 16;
 }
 
@@ -906,7 +764,8 @@ cudaError_t gru_persistent_forward(const GruDims& d, const float* const* w_hh, c
   p.y = y;
   p.rsv = (float4*)rsv;
   p.status = status;
-  return launch<false>(p, scratch, timeout_s, stream);
+  fill(p, scratch, timeout_s);
+  return launch_forward(p, stream);
 }
 
 cudaError_t gru_persistent_backward(const GruDims& d, const float* const* w_hh, const float* y, const float* rsv, const float* dy,
@@ -924,7 +783,8 @@ cudaError_t gru_persistent_backward(const GruDims& d, const float* const* w_hh, 
   p.dg = dg;
   p.db = db;
   p.status = status;
-  return launch<true>(p, scratch, timeout_s, stream);
+  fill(p, scratch, timeout_s);
+  return launch_backward(p, stream);
 }
 
 }  // namespace gpu
