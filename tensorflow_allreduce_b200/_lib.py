@@ -108,6 +108,8 @@ def _declare(lib):
         "bc_gru_scratch_bytes": (ll, [i, i, i, i]),
         "bc_gru_forward": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
         "bc_gru_backward": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
+        "bc_gru_forward_factors": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
+        "bc_gru_backward_factors": (i, [i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, d, vp]),
         "bc_conv_supported": (i, [i, P(i)]),
         "bc_conv_scratch_bytes": (ll, [P(i)]),
         "bc_bn_clip_forward": (i, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, f, f, vp]),

@@ -169,6 +169,11 @@ int bc_gru_forward(int T, int B, int H, int ndir, const float* w_hh0, const floa
                    const float* gx, float* y, float* rsv, void* scratch, unsigned* status, double timeout_s, void* stream);
 int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* y, const float* rsv,
                     const float* dy, float* dg, float* db, void* scratch, unsigned* status, double timeout_s, void* stream);
+/* The same with the factors of the backward pass, [ndir, T, B, 5, H], in the place of rsv: the faster pair. */
+int bc_gru_forward_factors(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* b_hh0, const float* b_hh1,
+                           const float* gx, float* y, float* fac, void* scratch, unsigned* status, double timeout_s, void* stream);
+int bc_gru_backward_factors(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* fac, const float* dy, float* dg,
+                            float* db, void* scratch, unsigned* status, double timeout_s, void* stream);
 
 /* Row convolutions (csrc/cuda/conv_rows.h): 32 output channels, stride (2, 1) with 32 input channels or (2, 2) with one.
  * `dims` = {N, Cin, H, W, KH, KW, ph, pw, stride_w}; `scratch` = bc_conv_scratch_bytes() bytes, contents irrelevant;

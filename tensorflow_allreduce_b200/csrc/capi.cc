@@ -575,7 +575,7 @@ int bc_gru_forward(int T, int B, int H, int ndir, const float* w_hh0, const floa
   gpu::GruDims d{T, B, H, ndir};
   const float* w[2] = {w_hh0, w_hh1};
   const float* b[2] = {b_hh0, b_hh1};
-  check_cuda(gpu::gru_persistent_forward(d, w, b, gx, y, rsv, scratch, status, timeout_s, (cudaStream_t)stream),
+  check_cuda(gpu::gru_persistent_forward(d, w, b, gx, y, rsv, nullptr, scratch, status, timeout_s, (cudaStream_t)stream),
              "persistent GRU forward launch");
   return 0;
   API_END(-1)
@@ -587,7 +587,32 @@ int bc_gru_backward(int T, int B, int H, int ndir, const float* w_hh0, const flo
   NvtxRange range("bcoll.gru_backward");
   gpu::GruDims d{T, B, H, ndir};
   const float* w[2] = {w_hh0, w_hh1};
-  check_cuda(gpu::gru_persistent_backward(d, w, y, rsv, dy, dg, db, scratch, status, timeout_s, (cudaStream_t)stream),
+  check_cuda(gpu::gru_persistent_backward(d, w, y, rsv, nullptr, dy, dg, db, scratch, status, timeout_s, (cudaStream_t)stream),
+             "persistent GRU backward launch");
+  return 0;
+  API_END(-1)
+}
+
+int bc_gru_forward_factors(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* b_hh0, const float* b_hh1,
+                           const float* gx, float* y, float* fac, void* scratch, unsigned* status, double timeout_s, void* stream) {
+  API_BEGIN
+  NvtxRange range("bcoll.gru_forward");
+  gpu::GruDims d{T, B, H, ndir};
+  const float* w[2] = {w_hh0, w_hh1};
+  const float* b[2] = {b_hh0, b_hh1};
+  check_cuda(gpu::gru_persistent_forward(d, w, b, gx, y, nullptr, fac, scratch, status, timeout_s, (cudaStream_t)stream),
+             "persistent GRU forward launch");
+  return 0;
+  API_END(-1)
+}
+
+int bc_gru_backward_factors(int T, int B, int H, int ndir, const float* w_hh0, const float* w_hh1, const float* fac, const float* dy, float* dg,
+                            float* db, void* scratch, unsigned* status, double timeout_s, void* stream) {
+  API_BEGIN
+  NvtxRange range("bcoll.gru_backward");
+  gpu::GruDims d{T, B, H, ndir};
+  const float* w[2] = {w_hh0, w_hh1};
+  check_cuda(gpu::gru_persistent_backward(d, w, nullptr, nullptr, fac, dy, dg, db, scratch, status, timeout_s, (cudaStream_t)stream),
              "persistent GRU backward launch");
   return 0;
   API_END(-1)

@@ -22,12 +22,12 @@ struct Params {
   const float* b_hh[2];   // forward: [3H] of each direction
   const float* gx;        // forward
   float* y;               // forward: out; backward: in (const)
-  float4* rsv;            // forward: out, or null; backward: in
+  float4* rsv;            // forward: out, or null; backward: in, where there are no factors
+  float* fac;             // forward: out, or null; backward: in, or null
   const float* dy;        // backward
   float* dg;              // backward: out
   float* db;              // backward: out
-  uint32_t* ring;         // operand words
-  uint4* xchg;            // backward, partial sums: [dir][owner block][source C][slot 2][pack][row] x 16 bytes
+  uint32_t* ring;         // what travels between blocks: operand words, behind them the partial sums of the backward pass
   uint32_t* sync;         // per direction: arrivals, generation
   uint32_t* status;
   unsigned long long timeout_ns;
@@ -67,6 +67,28 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, unsigned
   return true;
 }
 
+// The same for lanes that may have given up one by one.
+__device__ __forceinline__ bool lane_wait(uint32_t bar, uint32_t parity, unsigned long long timeout_ns, const volatile int* abort_flag) {
+  uint32_t spins = 0;
+  unsigned long long t0 = 0;
+  while (!mbar_try_wait(bar, parity)) {
+    if (((++spins) & 15) == 0) {
+      const unsigned long long now = gtimer();
+      if (t0 == 0) t0 = now;
+      if ((abort_flag && *abort_flag) || now - t0 > timeout_ns) return false;
+    }
+  }
+  return true;
+}
+
+// What dh is multiplied with to give the gradients of the pre-activations dr, dz, dn r and dn, and dh's share in the step before.
+struct Factors { float r, z, nr, n, keep; };
+// From r, z, n and hn = W_hn h + b_hn of a step and h of the step before.
+__device__ __forceinline__ Factors factors(float4 v, float hp) {
+  const float r = v.x, z = v.y, n = v.z, hn = v.w, c = (1.f - z) * (1.f - n * n);
+  return {c * hn * r * (1.f - r), (hp - n) * z * (1.f - z), c * r, c, z};
+}
+
 // The blocks of a direction meet once, at the start of a launch: thread 0 of each arrives, and leaves when all have.
 struct Meeting {
   uint32_t* count;
@@ -100,6 +122,7 @@ __device__ __forceinline__ bool meet_wait(const Params& p, const Meeting& m) {
 }
 
 cudaError_t launch_forward(const Params& p, cudaStream_t stream);
+cudaError_t launch_backward(const Params& p, cudaStream_t stream);
 
 }  // namespace gru
 }  // namespace gpu

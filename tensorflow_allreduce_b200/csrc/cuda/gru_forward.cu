@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_forward_kernel(const __grid_c
     const float* gx_p = p.gx + ((size_t)t_first * B + bb) * gx_row + dir * 3 * H + u0 + u;
     float* y_p = p.y + ((size_t)t_first * B + bb) * y_row + dir * H + u0 + u;
     float4* rsv_p = p.rsv ? p.rsv + ((size_t)(dir * T + t_first) * B + bb) * H + u0 + u : nullptr;
+    float* fac_p = p.fac ? p.fac + ((size_t)(dir * T + t_first) * B + bb) * 5 * H + u0 + u : nullptr;
     uint16_t* out = mine + bb * kKTile + u;
     const bool stamping = p.prof && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0;
     auto stamp = [&](int s, int i) {
@@ -463,6 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_forward_kernel(const __grid_c
         const float r_ = sigmoidf_(fmaf(acc[0], inv[0], gx[0] + bias[0]));
         const float z = sigmoidf_(fmaf(acc[1], inv[1], gx[1] + bias[1]));
         const float n = tanhf_(gx[2] + r_ * hn);
+        const float hp = h;
         h = n + z * (h - n);
         if (active) {
           if (s + 1 < T) st_half(out + ((s & 1) ? slot_halves : 0u), tagged_half(h, phase ^ (uint32_t)(u & 1)));
@@ -470,9 +472,14 @@ __global__ void __launch_bounds__(kThreads, 1) gru_forward_kernel(const __grid_c
           // The other blocks do not wait for what follows.
           *y_p = h;
           if (rsv_p) *rsv_p = make_float4(r_, z, n, hn);
+          if (fac_p) {
+            const Factors f = factors(make_float4(r_, z, n, hn), hp);
+            fac_p[0] = f.r; fac_p[H] = f.z; fac_p[2 * H] = f.nr; fac_p[3 * H] = f.n; fac_p[4 * H] = f.keep;
+          }
         }
         y_p += step * B * y_row;
         if (rsv_p) rsv_p += step * B * H;
+        if (fac_p) fac_p += step * B * 5 * H;
         if (s + 1 < T) load_gx();
       }
       if (s + 1 == T) break;

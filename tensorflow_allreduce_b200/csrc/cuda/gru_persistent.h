@@ -34,29 +34,32 @@ constexpr uint32_t kGruTimeoutGrid = 1u;      // waiting for the other blocks of
 constexpr uint32_t kGruTimeoutBlock = 2u;     // waiting for other warps of the block
 constexpr uint32_t kGruTimeoutMma = 4u;       // waiting for the tensor core to finish
 
-// Forward. All tensors are fp32, contiguous, on the current device; w_hh, rsv and scratch 16-byte aligned.
+// Forward. All tensors are fp32, contiguous, on the current device; w_hh, rsv, fac and scratch 16-byte aligned.
 //   w_hh[dir] [3H, H]          recurrent weights of each direction
 //   b_hh[dir] [3H]
 //   gx    [T, B, ndir, 3H]     input projections including b_ih
 //   y     [T, B, ndir*H]       output
-//   rsv   [ndir, T, B, H, 4]   r, z, n and (W_hn h + b_hn) of every step, for the backward pass; may be null
+// For the backward pass, one of these or none:
+//   rsv   [ndir, T, B, H, 4]   r, z, n and (W_hn h + b_hn) of every step
+//   fac   [ndir, T, B, 5, H]   what dh is multiplied with to give dr, dz, dn r, dn and its share in the step before
 //   scratch                    gru_persistent_scratch_bytes(d) bytes, zeroed once when they are allocated and then reused
 //                              as they are by later calls, one after the other (concurrent calls need one each)
 //   status[1] uint32           ORed with kGruTimeout* on failure
 // `timeout_s` bounds every wait inside the kernel. Returns cudaErrorInvalidValue for unsupported
 // dimensions and cudaErrorCooperativeLaunchTooLarge if the grid cannot be co-resident.
 cudaError_t gru_persistent_forward(const GruDims& d, const float* const* w_hh, const float* const* b_hh, const float* gx, float* y,
-                                   float* rsv, void* scratch, uint32_t* status, double timeout_s, cudaStream_t stream);
+                                   float* rsv, float* fac, void* scratch, uint32_t* status, double timeout_s, cudaStream_t stream);
 
 // Backward through time.
-//   y, rsv                     from the forward pass
+//   y, rsv or fac              from the forward pass; `fac` is the faster one (dh travels between the blocks instead of three gradients either way,
+//                              but with `rsv` every block of a group forms the factors of its whole range), y is not read beside it
 //   dy     [T, B, ndir*H]      gradient of the output
 //   dg     [T, B, ndir*4H]     out: gradients of the pre-activations. Columns [0, ndir*3H): those of gx, (dr, dz, dn) of
 //                              direction 0, then of direction 1; columns ndir*3H + dir*H: dn * r. The gradient of
 //                              (W_h h + b_h) is (dr, dz, dn * r), so the two share their first two parts.
 //   db     [ndir, 2, 3H]       out: sums over time and batch of (dr, dz, dn) and of (dr, dz, dn * r): gradients of b_ih and b_hh
 // The caller forms dW_ih, dx and dW_hh from dg with library GEMMs.
-cudaError_t gru_persistent_backward(const GruDims& d, const float* const* w_hh, const float* y, const float* rsv, const float* dy,
+cudaError_t gru_persistent_backward(const GruDims& d, const float* const* w_hh, const float* y, const float* rsv, const float* fac, const float* dy,
                                     float* dg, float* db, void* scratch, uint32_t* status, double timeout_s, cudaStream_t stream);
 
 // An upper bound of the bytes of partial sums (plain fp32) that one step exchanges, and the bytes of scratch memory that a forward or

@@ -170,7 +170,7 @@ Tensor aligned(const Tensor& t) {
   return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) == 0 ? c : c.clone();
 }
 
-// One layer: output, and what its backward pass needs (x, all input weights, y, saved activations, recurrent weights).
+// One layer: output, and what its backward pass needs (x, all input weights, y, factors of dh, recurrent weights).
 // `w` holds w_ih, w_hh, b_ih, b_hh of every direction.
 Tensor gru_run(const Tensor& x, at::TensorList w, bool save, variable_list* keep) {
   const int64_t T = x.size(0), B = x.size(1), I = x.size(2), nd = (int64_t)w.size() / 4, H = w[1].size(1);
@@ -183,16 +183,16 @@ Tensor gru_run(const Tensor& x, at::TensorList w, bool save, variable_list* keep
   // input projections of both directions in one GEMM: [T*B, nd*3H]
   const Tensor gx = at::addmm(b_ih, x.reshape({T * B, I}), w_ih.t());
   Tensor y = at::empty({T, B, nd * H}, x.options());
-  Tensor rsv;
-  if (save) rsv = at::empty({nd, T, B, H, 4}, x.options());
+  Tensor fac;
+  if (save) fac = at::empty({nd, T, B, 5, H}, x.options());
   void* s = stream_of(x);
   const Tensor scratch = gru_scratch(x, s, T, B, H, nd);
-  check(bc_gru_forward((int)T, (int)B, (int)H, (int)nd, ptr(w_hh[0]), ptr(w_hh[nd - 1]), ptr(b_hh[0]), ptr(b_hh[nd - 1]), ptr(gx), ptr(y), ptr(rsv),
-                       scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, s),
-        "bc_gru_forward");
+  check(bc_gru_forward_factors((int)T, (int)B, (int)H, (int)nd, ptr(w_hh[0]), ptr(w_hh[nd - 1]), ptr(b_hh[0]), ptr(b_hh[nd - 1]), ptr(gx), ptr(y),
+                               ptr(fac), scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, s),
+        "bc_gru_forward_factors");
   g_gru_launches++;
   if (save) {
-    *keep = {x, w_ih, y, rsv, w_hh[0]};
+    *keep = {x, w_ih, y, fac, w_hh[0]};
     if (nd > 1) keep->push_back(w_hh[1]);
   }
   return y;
@@ -209,7 +209,7 @@ struct GruLayer : torch::autograd::Function<GruLayer> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w_ih = saved[1], &y = saved[2], &rsv = saved[3];
+    const Tensor &x = saved[0], &w_ih = saved[1], &y = saved[2], &fac = saved[3];
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t nd = (int64_t)saved.size() - 4, T = x.size(0), B = x.size(1), I = x.size(2), H = saved[4].size(1), H3 = 3 * H;
     const Tensor dy = grads[0].contiguous();
@@ -217,9 +217,9 @@ struct GruLayer : torch::autograd::Function<GruLayer> {
     Tensor dg = at::empty({T * B, nd * 4 * H}, x.options()), db = at::empty({nd, 2, H3}, x.options());
     void* s = stream_of(x);
     const Tensor scratch = gru_scratch(x, s, T, B, H, nd);
-    check(bc_gru_backward((int)T, (int)B, (int)H, (int)nd, ptr(saved[4]), ptr(saved[3 + nd]), ptr(y), ptr(rsv), ptr(dy), ptr(dg), ptr(db),
-                          scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, s),
-          "bc_gru_backward");
+    check(bc_gru_backward_factors((int)T, (int)B, (int)H, (int)nd, ptr(saved[4]), ptr(saved[3 + nd]), ptr(fac), ptr(dy), ptr(dg), ptr(db),
+                                  scratch.data_ptr(), (unsigned*)gru_status(x), g_gru_timeout_s, s),
+          "bc_gru_backward_factors");
     g_gru_launches++;
     const Tensor dgx = dg.narrow(1, 0, nd * H3);
     variable_list out(1 + 4 * nd);

@@ -42,3 +42,16 @@ def test_scratch_holds_what_the_kernels_address(native_lib):
                     assert nd * 2 * C * -(-kq // 32) * nb * 32 * 4 <= ring
                     need = max(need, nd * blocks * C * 2 * -(-B // 3) * rows * 16)
                 assert native_lib.bc_gru_scratch_bytes(7, B, H, nd) == 1024 + ring + need
+
+
+def test_partial_sums_of_the_backward_pass_fit_behind_its_ring(native_lib):
+    # Restated from gru_backward.cu: groups of C blocks, a ring of [direction][slot][member][tile of 32 units][batch 16 or 32][32] words, behind it
+    # [direction][owner block][source, without the owner][slot][pack of three][row] words of 16 bytes.
+    for nd in (1, 2):
+        for H in range(128, 1025, 128):
+            for B in range(1, 33):
+                nb = 16 if B <= 16 else 32
+                C = 4 if nb == 32 and H <= 256 else 8
+                ring = nd * 2 * C * -(-H // C // 32) * nb * 32 * 4
+                sums = nd * (H // 16) * (C - 1) * 2 * -(-B // 3) * 16 * 16
+                assert 1024 + ring + sums <= native_lib.bc_gru_scratch_bytes(7, B, H, nd)
