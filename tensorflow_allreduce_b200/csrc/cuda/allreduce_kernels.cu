@@ -24,6 +24,7 @@
 #include "device_prims.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 namespace bc {
@@ -555,14 +556,16 @@ cudaError_t launch_copy(void* dst, const void* src, size_t bytes, cudaStream_t s
   if ((((uintptr_t)dst | (uintptr_t)src) & 15) != 0) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s);
   const size_t npacks = bytes / 16;
   const int ntail = (int)(bytes % 16);
-  // At most 592 blocks, four per SM of a B200. One load per thread while all of them are in flight at once anyway, so that a small tensor
-  // is spread over as many SMs as it has blocks; eight for tensors of several passes. us with 1 / 4 / 8 loads: 40 KB 3.87 / 4.24 / 4.24
-  // (a launch by itself takes about 3.8), 1 MB 4.23 / 4.23 / 4.29, 4.8 MB 5.40 / 4.97 / 5.79, 12 MB 8.32 / 7.19 / 7.65,
-  // 19 MB 10.8 / 9.35 / 9.56, 25 MB 12.8 / 11.3 / 11.3, 64 MB 25.2 / 25.2 / 24.6, 256 MB 92.9 / 93.7 / 87.0 (twice the blocks: 84.5).
+  // One load per thread while 592 blocks, four per SM of a B200, hold all of it, so that a small tensor is spread over as many SMs as it has
+  // blocks; eight for tensors of several times as much. us with 1 / 4 / 8 loads: 40 KB 3.87 / 4.24 / 4.24 (a launch by itself takes about 3.8),
+  // 1 MB 4.23 / 4.23 / 4.29, 4.8 MB 5.40 / 4.97 / 5.79, 12 MB 8.32 / 7.19 / 7.65, 19 MB 10.8 / 9.35 / 9.56, 25 MB 12.8 / 11.3 / 11.3.
+  // Large tensors have a block for every run of eight loads, not 592 that go through the tensor in step: those that finish early make room for the next, and
+  // reads and writes of neighbouring rows of memory stay closer together. us with 592 / 1184 / 2368 blocks / one per run: 64 MB 24.8 / 23.7 /
+  // 23.7 / 24.1, 128 MB 43.1 / 44.0 / 37.8 / 37.7, 256 MB 86.5 / 80.2 / 83.1 / 82.8, 512 MB 172.5 / 166.9 / 164.1 / 159.9. 32-byte accesses are no faster.
   const size_t kOnePass = 592u * kCopyThreads;
   const int unroll = npacks <= kOnePass ? 1 : npacks <= 4 * kOnePass ? 4 : 8;
   const size_t run = (size_t)kCopyThreads * unroll;
-  const int blocks = (int)std::max<size_t>(1, std::min<size_t>((npacks + run - 1) / run, 592));
+  const int blocks = (int)std::max<size_t>(1, std::min<size_t>((npacks + run - 1) / run, INT_MAX));
   auto kernel = unroll == 1 ? copy_kernel<1> : unroll == 4 ? copy_kernel<4> : copy_kernel<8>;
   kernel<<<blocks, kCopyThreads, 0, s>>>((uint4*)dst, (const uint4*)src, npacks, (char*)dst + npacks * 16,
                                      (const char*)src + npacks * 16, ntail);
