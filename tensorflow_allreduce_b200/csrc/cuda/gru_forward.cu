@@ -95,10 +95,6 @@ __device__ __forceinline__ float tanhf_(float x) {
 // whatever waits have run out.
 __device__ __forceinline__ void group_sync(int group) { asm volatile("barrier.cta.sync %0, 128;" ::"r"(group + 1) : "memory"); }
 
-// 16 bytes from global to shared memory, asynchronously.
-__device__ __forceinline__ void copy16(float* to, const float* from) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to)), "l"(from) : "memory"); }
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // ---- fp16 operands -------------------------------------------------------------------------------
 
 __device__ __forceinline__ uint16_t half_rn(float v) {
@@ -214,13 +210,8 @@ struct Plan {
   static constexpr int kParts = std::min(kRounds, kMaxParts);               // what is handed to the tensor core at a time
   static constexpr int kRoundsPerPart = (kRounds + kParts - 1) / kParts;
   static constexpr int kXBytes = kTiles * kTileBytes, kWBytes = (kTiles - kTmemTiles) * kRows * 128;
-  // The 48 rows of weights as they are, at the start, and in their place the operand and the read-back of the warps; weights, scales of the rows,
-  // barriers.
-  static constexpr int kStageRow = H + 4;                                    // floats; the four keep rows in different banks
-  static constexpr int kBackAt = kXBytes, kStageBytes = 3 * kUnits * kStageRow * 4;
-  static constexpr int kWAt = (std::max(kBackAt + kWarps / 4 * kBackGroup * 4, kStageBytes) + 1023) / 1024 * 1024;
-  static constexpr int kSmem = 1024 + kWAt + kWBytes + 256 + 128;
-  static_assert(kSmem <= 227 * 1024, "");
+  // operand, weights, read-back of the warps, scales of the 48 rows, barriers
+  static constexpr int kSmem = 1024 + kXBytes + kWBytes + kWarps / 4 * kBackGroup * 4 + 256 + 128;
 };
 
 // Sixteen weights of a row times its scale as pairs of fp16: the upper part, or what it leaves.
@@ -228,7 +219,7 @@ __device__ __forceinline__ void split16(const float* p, float scale, bool lower,
   uint16_t h[16];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const float4 f = reinterpret_cast<const float4*>(p)[i];
+    const float4 f = __ldg(reinterpret_cast<const float4*>(p) + i);
     const float v[4] = {f.x * scale, f.y * scale, f.z * scale, f.w * scale};
 #pragma unroll
     for (int e = 0; e < 4; e++) {
@@ -257,26 +248,15 @@ __global__ void __launch_bounds__(kThreads, 1) gru_forward_kernel(const __grid_c
   const int rank = CTAS == 1 ? 0 : blockIdx.x & 1;
 
   uint8_t* x_s = smem;
-  float* stage_s = reinterpret_cast<float*>(smem);
-  float* back_s = reinterpret_cast<float*>(smem + pl::kBackAt);        // read-back
-  uint8_t* w_s = smem + pl::kWAt;
-  float* scale_s = reinterpret_cast<float*>(w_s + pl::kWBytes);        // [gate][unit]: power of two of each row
+  uint8_t* w_s = x_s + pl::kXBytes;
+  float* back_s = reinterpret_cast<float*>(w_s + pl::kWBytes);          // read-back
+  float* scale_s = back_s + kWarps / 4 * kBackGroup;                              // [gate][unit]: power of two of each row
   uint64_t* bar_s = reinterpret_cast<uint64_t*>(scale_s + 64);         // full[kMaxParts], done, drain
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_s + kMaxParts + 2);
   volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t full_bar = smem_u32(bar_s), done_bar = full_bar + 8 * kMaxParts, drain_bar = done_bar + 8;
   const uint32_t x_addr = smem_u32(x_s), w_addr = smem_u32(w_s);
 
-  // The weights of the block's 48 rows, three rows per warp.
-  const float* w = p.w_hh[dir];
-  if (warp < kWarps)
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const int r = 3 * warp + k;
-      const float* row = w + (size_t)(r / kUnits * H + u0 + r % kUnits) * H;
-#pragma unroll
-      for (int i = 0; i < H / 128; i++) copy16(stage_s + r * pl::kStageRow + 4 * lane + 128 * i, row + 4 * lane + 128 * i);
-    }
   if (tid == 0) {
     for (int i = 0; i < kMaxParts; i++) mbar_init(full_bar + 8 * i, kWarps + (rank == 0 ? CTAS - 1 : 0));
     mbar_init(done_bar, 1);
@@ -292,25 +272,27 @@ __global__ void __launch_bounds__(kThreads, 1) gru_forward_kernel(const __grid_c
   uint16_t* mine = ring + (size_t)(u0 / kKTile) * NB * kKTile + u0 % kKTile;
   for (int i = tid; i < 2 * B * kUnits; i += kThreads)
     st_half(mine + (i & 1 ? slot_halves : 0u) + (i / 2 / kUnits) * kKTile + i / 2 % kUnits, 0);
+  for (int i = tid; i < pl::kXBytes / 16; i += kThreads) reinterpret_cast<uint4*>(x_s)[i] = make_uint4(0, 0, 0, 0);
 
   // Scale of every row. Infinite weights and NaN are left out of the maximum: they stay what they are.
-  if (warp < kWarps) {
-    copies_wait();
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const int r = 3 * warp + k;
+  const float* w = p.w_hh[dir];
+  if (warp < kWarps)
+    for (int r = warp; r < 3 * kUnits; r += kWarps) {
+      const float4* row = reinterpret_cast<const float4*>(w + (size_t)(r / kUnits * H + u0 + r % kUnits) * H);
       uint32_t m = 0;
+      for (int i = lane; i < H / 4; i += 32) {
+        const float4 v = __ldg(row + i);
+        const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int i = 0; i < H / 32; i++) {
-        const uint32_t b = __float_as_uint(stage_s[r * pl::kStageRow + lane + 32 * i]) & 0x7FFFFFFFu;
-        if (b < 0x7F800000u) m = max(m, b);
+        for (int e = 0; e < 4; e++) {
+          const uint32_t b = __float_as_uint(f[e]) & 0x7FFFFFFFu;
+          if (b < 0x7F800000u) m = max(m, b);
+        }
       }
       m = __reduce_max_sync(0xffffffffu, m);
       const int e = m ? max((int)(m >> 23) - 127, -90) : 14;
       if (lane == 0) scale_s[r] = pow2(14 - e);
     }
-  }
   fence_proxy_async();
   __threadfence();
   tc_fence_before();
@@ -326,7 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1) gru_forward_kernel(const __grid_c
   if (warp < kWarps) {
     const bool row_ok = gate < 3;
     const int unit = 4 * quarter + (lane & 3);
-    const float* row = stage_s + ((row_ok ? gate : 0) * kUnits + unit) * pl::kStageRow;
+    const float* row = w + (size_t)((row_ok ? gate : 0) * H + u0 + unit) * H;
     const float scale = row_ok ? scale_s[gate * kUnits + unit] : 0.f;
     for (int kt = warp >> 2; kt < pl::kTiles; kt += kWarps / 4) {
       uint32_t v[32];
@@ -414,14 +396,6 @@ __global__ void __launch_bounds__(kThreads, 1) gru_forward_kernel(const __grid_c
     const uint32_t* src0 = reinterpret_cast<const uint32_t*>(ring) + (size_t)(kt0 * NB + xb) * (kKTile / 2) + sector * 8;
     constexpr uint32_t kRoundBytes = kWorkers * 32, kRoundWords = pl::kTilesPerRound * NB * kKTile / 2;   // in shared memory, in the ring
     const int loads = xb < B && kt0 < pl::kTiles ? (pl::kTiles - kt0 + pl::kTilesPerRound - 1) / pl::kTilesPerRound : 0;
-
-    // Operand rows without a batch entry are zero: each thread clears those that it would load. (The weights have been taken from here.)
-    if (xb >= B) {
-      const Words zero = {};
-      for (int i = 0; i < pl::kRounds; i++)
-        if (kt0 + i * pl::kTilesPerRound < pl::kTiles) st_shared2(dst + i * kRoundBytes, zero);
-      fence_proxy_async();
-    }
 
     // Gates: unit u of the block, batch entry b. The four warps of a column group read eight columns back, each those of its quarter of the
     // rows, and share them through shared memory. The next step writes those only when all warps have brought their words of it.
