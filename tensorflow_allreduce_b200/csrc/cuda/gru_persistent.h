@@ -1,8 +1,7 @@
 // Persistent bidirectional GRU layer for sm_100a: the recurrent weights of a layer stay on chip (tensor
 // memory, and shared memory for what does not fit) for all time steps, the per-step recurrent product runs
-// on the 5th-generation tensor cores (tcgen05.mma, TF32 operands, fp32 accumulator), groups of blocks split
-// the reduction length of the product among themselves, and the two directions run side by side in one
-// cooperative launch.
+// on the 5th-generation tensor cores (tcgen05.mma, fp16 pairs forward, TF32 backward, fp32 accumulator), and the
+// two directions run side by side in one cooperative launch. gru_forward.cu, gru_backward.cu: the kernels.
 //
 // The reference's speech-model pieces are GRU cells that launch one GEMM plus elementwise
 // kernels per time step (tensorflow/contrib/rnn/kernels/gru_ops.h:69-119, gru_ops_gpu.cu.cc) or
@@ -68,8 +67,8 @@ size_t gru_persistent_workspace_bytes(const GruDims& d);
 size_t gru_persistent_scratch_bytes(const GruDims& d);
 
 // Tuning aid: when `stamps` (device memory, 8 x T uint64) is non-null, thread 0 of block (0, 0) of every later
-// launch records %globaltimer at fixed points of each step: [0] step start, [1] operand in shared memory, [2] accumulator
-// complete, [3] partial sums sent, [4] partial sums received, [5] step published. Null switches it off.
+// launch records %globaltimer at fixed points of each step. Forward: [0] step start, [1] accumulator complete, [2] read back, [3] published, [4] outputs stored, [5] paused,
+// [6] its words in shared memory. Backward: [0] step start, [4] published, [1] accumulator complete, [2] partial sums sent, [3] received. Null switches it off.
 void gru_persistent_set_profile(unsigned long long* stamps);
 
 // True if this device and these dimensions can run the persistent kernels.

@@ -1,4 +1,4 @@
-"""Persistent GRU layers on the tcgen05 kernels of `csrc/cuda/gru_persistent.cu`.
+"""Persistent GRU layers on the tcgen05 kernels of `csrc/cuda/gru_forward.cu` and `gru_backward.cu`.
 
 A GRU layer is split the usual way into the input projections of all time steps (one library
 GEMM) and the recurrence. The recurrence of both directions of a layer runs in ONE cooperative
