@@ -16,7 +16,7 @@ bool dims_ok(const GruDims& d) {
   return d.T >= 1 && d.T < 4096 && d.B >= 1 && d.B <= 32 && d.H >= 128 && d.H <= 1024 && d.H % 128 == 0 && (d.ndir == 1 || d.ndir == 2);
 }
 
-bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+bool aligned(const void* p, uintptr_t bytes) { return ((uintptr_t)p & (bytes - 1)) == 0; }
 
 // Bytes of partial sums (fp32, 32 batch rows, a block's own included) of a step with groups of 4 blocks forward and 16 backward, wider
 // than any that is launched.
@@ -35,10 +35,11 @@ int exchange_rows(const GruDims& d) {
 }
 
 cudaError_t start(Params& p, const GruDims& d, const float* const* w_hh, void* scratch, uint32_t* status, double timeout_s) {
-  if (!dims_ok(d) || !aligned16(p.rsv) || !aligned16(p.fac) || !aligned16(scratch)) return cudaErrorInvalidValue;
+  // factors and words of the ring are read 32 bytes at a time
+  if (!dims_ok(d) || !aligned(p.rsv, 16) || !aligned(p.fac, 32) || !aligned(scratch, 32)) return cudaErrorInvalidValue;
   p.d = d;
   for (int i = 0; i < d.ndir; i++) {
-    if (!aligned16(w_hh[i])) return cudaErrorInvalidValue;
+    if (!aligned(w_hh[i], 16)) return cudaErrorInvalidValue;
     p.w_hh[i] = w_hh[i];
   }
   char* w = (char*)scratch;

@@ -165,9 +165,9 @@ Tensor gru_scratch(const Tensor& like, void* stream, int64_t T, int64_t B, int64
   return t;
 }
 
-Tensor aligned(const Tensor& t) {
+Tensor aligned(const Tensor& t, uintptr_t bytes = 16) {
   Tensor c = t.contiguous();
-  return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) == 0 ? c : c.clone();
+  return (reinterpret_cast<uintptr_t>(c.data_ptr()) & (bytes - 1)) == 0 ? c : c.clone();
 }
 
 // One layer: output, and what its backward pass needs (x, all input weights, y, factors of dh, recurrent weights).
@@ -209,10 +209,10 @@ struct GruLayer : torch::autograd::Function<GruLayer> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w_ih = saved[1], &y = saved[2], &fac = saved[3];
+    const Tensor &x = saved[0], &w_ih = saved[1], &y = saved[2];
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t nd = (int64_t)saved.size() - 4, T = x.size(0), B = x.size(1), I = x.size(2), H = saved[4].size(1), H3 = 3 * H;
-    const Tensor dy = grads[0].contiguous();
+    const Tensor dy = grads[0].contiguous(), fac = aligned(saved[3], 32);      // hooks of saved tensors may return views
     // gradients of the pre-activations: (dr, dz, dn) of every direction, then dn * r of every direction
     Tensor dg = at::empty({T * B, nd * 4 * H}, x.options()), db = at::empty({nd, 2, H3}, x.options());
     void* s = stream_of(x);

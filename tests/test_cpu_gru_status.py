@@ -1,5 +1,6 @@
 """The host side of the persistent GRU layers without a GPU: what `persistent_gru.check_status` makes of the status words (the extension is a
 stand-in), the size of the memory through which blocks exchange."""
+import ctypes
 import types
 
 import pytest
@@ -55,3 +56,18 @@ def test_partial_sums_of_the_backward_pass_fit_behind_its_ring(native_lib):
                 ring = nd * 2 * C * -(-H // C // 32) * nb * 32 * 4
                 sums = nd * (H // 16) * (C - 1) * 2 * -(-B // 3) * 16 * 16
                 assert 1024 + ring + sums <= native_lib.bc_gru_scratch_bytes(7, B, H, nd)
+
+
+def test_alignment_is_refused_before_a_launch(native_lib):
+    # The kernels read factors and exchange memory 32 bytes at a time. Nothing is dereferenced: without a GPU an aligned call ends at the device.
+    from tensorflow_allreduce_b200 import _lib
+
+    p = lambda at: ctypes.c_void_p(at)
+    base = 1 << 20
+    for fac, scratch in ((base + 16, base), (base, base + 16), (base + 4, base)):
+        with pytest.raises(Exception, match="invalid argument"):
+            _lib.check(native_lib.bc_gru_backward_factors(3, 2, 128, 1, p(base), p(base), p(fac), p(base), p(base), p(base), p(scratch), p(base), 1.0,
+                                                          p(None)), "backward")
+        with pytest.raises(Exception, match="invalid argument"):
+            _lib.check(native_lib.bc_gru_forward_factors(3, 2, 128, 1, p(base), p(base), p(base), p(base), p(base), p(base), p(fac), p(scratch), p(base),
+                                                         1.0, p(None)), "forward")
